@@ -20,7 +20,7 @@ BUILD = os.path.join(HERE, "_build")
 LIB = os.path.join(HERE, "libaerocfd_gpu.so")
 INCLUDE = os.path.join(os.path.dirname(HERE), "include")
 
-SOURCES = ["aero_flux.cu", "aero_implicit.cu", "aero_bc.cu", "aero_transfer.cu",
+SOURCES = ["aero_flux.cu", "aero_implicit.cu", "aero_pipe.cu", "aero_bc.cu", "aero_transfer.cu",
            "aero_runtime.cu", "aero_topology.cpp", "aero_geometry.cu", "aero_sa.cu",
            "aero_noalloc.cu", "aero_forces.cu", "aero_crank.cu", "aero_mlp.cu", "aero_crmath.cu"]
 HEADERS = ["aero_device.cuh", "aero_kernels.h", "aero_topology.h", "aero_mlp_gemm.cuh", "aero_crmath.h",

@@ -55,6 +55,51 @@ struct CaseConsts {
   int inviscid;  // iflag_inviscid: 4 Roe + WENO3, 5 Steger-Warming + WENO5, 8 WCNS5 + Roe
 };
 
+// The pipelined sweeps' view of a block (aero_pipe.cu).  The updated box is cut
+// along direction `dir` into `ce` slabs, slab r holding the offsets
+// [r*n/ce, (r+1)*n/ce) of that direction's n.  Every slab has its own
+// hyperplanes (sums of the node's offsets inside the slab); the positions list
+// the nodes slab by slab, plane by plane, and inside a plane by the k-offset,
+// then the j-offset.
+struct PipePlane {
+  int pos, cnt;  // first position, nodes
+};
+struct PipeView {
+  int dir, ce;
+  int* slab;         // ce+1: first entry of each slab in `plane`
+  PipePlane* plane;
+  int* at;           // per updated node in box order: its position
+  double* rec;       // kPipeRec words per position
+  double* sa_rec;    // kPipeSaRec words per position
+};
+// One node's record, 336 bytes: the words of one plane are one chunk for the
+// bulk copies, a thread reads its node's words in 16-byte pairs at fixed
+// offsets, and the stride (80 bytes past a multiple of 128) puts eight
+// neighbouring nodes' pairs into different banks.
+constexpr int kPipeRec = 42;
+enum PipeWord {
+  PW_M = 0,     // rho*u, rho*v, rho*w, rho
+  PW_RCP = 4,   // 1/rho in two words (a NaN: IEEE divisions)
+  PW_PHI = 6,   // calc_jm's phi and a1
+  PW_DIR = 8,   // per direction 6 words: U, its three metrics, its radius, 0.5*inv_j
+  PW_NBR = 26,  // the neighbour word
+  PW_DIV = 28,  // diag, inv_j, 1/diag, 1/inv_j, the low words of both reciprocals
+  PW_RHS = 34,  // rhs, then dq*, then dq (5)
+  PW_OK = 39    // 1 or 0: both divisors in div2_pair's range
+};
+
+// The SA equation's record, 112 bytes (16 short of a multiple of 128: as above).
+constexpr int kPipeSaRec = 14;
+enum SaWord {
+  SW_A = 0,    // upwind coefficients of the i-1, j-1, k-1 neighbours
+  SW_NBR = 3,  // the neighbour word
+  SW_B = 4,    // of the i+1, j+1, k+1 neighbours
+  SW_NAT = 7,  // natural (box) index
+  SW_RHS = 8,  // sa_rhs, then dnut*; diag, 1/diag in two words
+  SW_NUT = 12,
+  SW_OK = 13   // 1 or 0: the diagonal in div2_pair's range
+};
+
 // Everything a kernel needs to address one block's fields.
 struct BlockView {
   Box b, b0, b1;
@@ -80,6 +125,7 @@ struct BlockView {
   double* sa_dq;         // 1 per node: SA forward-sweep increment
   double* dqs;           // 8 per node: dq* (forward result), padded to 64 bytes
   double* dq;            // 5 per node: dq (backward result)
+  PipeView pipe;         // the pipelined sweeps' order and records
   // Case constants of this block when blocks of different cases share one
   // launch (a batch); nullptr: the launch's constants apply.
   const CaseConsts* ccb;
@@ -211,6 +257,29 @@ __device__ __forceinline__ double div2_rn(double a, double b1, double rb1, doubl
   double q = div_newton(div_newton(a, b1, rb1), b2, rb2);
   const double aa = fabs(a);
   if (!(bok && aa > 0x1p-500 && aa < 0x1p500)) q = div2_ieee(a, b1, b2);
+  return q;
+}
+
+// a / b from the reciprocal of b in two words, rh = 1/b rounded and
+// rl = (1 - b*rh)*rh rounded (recip_lo): a*rh + a*rl, the product with rh
+// rounded once with the other added, is a/b within far less than an ulp, so one
+// of Markstein's corrections rounds it correctly.  The same bits as
+// div_newton with one operation less, under the same conditions on the ranges
+// (and a = 0 loses its sign).
+__device__ __forceinline__ double recip_lo(double b, double rh) { return fma(-b, rh, 1.0) * rh; }
+__device__ __forceinline__ double div_pair(double a, double b, double rh, double rl) {
+  double q = fma(a, rh, a * rl);
+  double r = fma(-q, b, a);
+  return fma(r, rh, q);
+}
+// div2_rn with both reciprocals in two words: (a / b1) / b2, bit for bit but
+// for a = 0, which gives +0 whatever the signs (div2_rn's IEEE path is a call;
+// the spanwise row of a flow without spanwise velocity is 0 at every node).
+__device__ __forceinline__ double div2_pair(double a, double b1, double rh1, double rl1, double b2, double rh2,
+                                            double rl2, bool bok) {
+  double q = div_pair(div_pair(a, b1, rh1, rl1), b2, rh2, rl2);
+  const double aa = fabs(a);
+  if (!(bok && (aa > 0x1p-500 || a == 0.0) && aa < 0x1p500)) q = div2_ieee(a, b1, b2);
   return q;
 }
 

@@ -103,6 +103,47 @@ __global__ void k_lusgs_sca_f32(const BlockView* __restrict__ blocks);
 __global__ void k_plane_index(const BlockView* __restrict__ blocks);
 __global__ void k_lusgs_mats(const BlockView* __restrict__ blocks, CaseConsts cc);
 __global__ void k_lusgs_mats_f32(const BlockView* __restrict__ blocks, CaseConsts cc);
+// pipelined sweeps (aero_pipe.cu).  Launch shape: P nodes of a plane at most, NG
+// groups of W warps, NST stages, D inbox slots (a power of two) of L nodes' values.
+struct PipeShape {
+  int P, W, NG, NST, D, L;
+};
+// words of a node's products between the planes
+constexpr int kPipeProd = 17;
+// Dynamic shared memory of a launch, in 8-byte words from the start: 16 zeros and
+// 16 words nobody reads, NST stages of P records, two planes of P nodes'
+// products, D messages, 2*NST + D + 1 mbarriers, a slab's planes (at most H).
+struct PipeSmem {
+  int stage, ring, inbox, bars, planes, words;
+  // rec, prod, val: words of a record, of a node's products, of a message's node
+  __host__ __device__ PipeSmem(const PipeShape& s, int rec, int prod, int val, int H) {
+    stage = 32;
+    ring = stage + s.NST * s.P * rec;
+    inbox = ring + 2 * prod * s.P;
+    bars = inbox + s.D * val * s.L;
+    planes = bars + 2 * s.NST + s.D + 1;
+    words = planes + H;
+  }
+};
+// a poll budget of this many polls means the time bound of the cluster waits
+constexpr long kPipePolls = 1L << 20;
+__global__ void k_pipe_index(const BlockView* __restrict__ blocks);
+__global__ void k_pipe_recs(const BlockView* __restrict__ blocks, CaseConsts cc);
+__global__ void k_pipe_sca(const BlockView* __restrict__ blocks, CaseConsts cc);
+__global__ void k_pipe_update(const BlockView* __restrict__ blocks);
+// The sweeps, FP64 or with the blocks rounded to FP32 (mixed precision), for CTAs
+// of at most kPipeWarps[variant] warps, kPipeCtas[variant] of them per SM: fewer
+// warps have more registers each, in which a thread's 25 block entries are
+// formed with more operations in flight.
+constexpr int kPipeVariants = 5;
+constexpr int kPipeWarps[kPipeVariants] = {8, 11, 16, 6, 8};
+constexpr int kPipeCtas[kPipeVariants] = {1, 1, 1, 2, 2};
+using PipeKernel = void (*)(const BlockView*, CaseConsts, PipeShape, unsigned*, long, int);
+PipeKernel pipe_kernel(int variant, bool f32);
+// the same for the SA equation
+__global__ void k_pipe_sa_recs(const BlockView* __restrict__ blocks, CaseConsts cc);
+__global__ void k_pipe_sa_sweep(const BlockView* __restrict__ blocks, CaseConsts cc, PipeShape sh, unsigned* status,
+                                long spin_limit, int stall_plane);
 __global__ void k_sa_length(const BlockView* __restrict__ blocks, CaseConsts cc);
 __global__ void k_sa_a(const BlockView* __restrict__ blocks, CaseConsts cc);
 __global__ void k_sa_b(const BlockView* __restrict__ blocks, CaseConsts cc);

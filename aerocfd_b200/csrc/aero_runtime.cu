@@ -25,6 +25,9 @@ using namespace aero;
 
 namespace {
 
+// Streaming multiprocessors of the device the launch shapes are made for.
+constexpr int kSms = 148;
+
 struct HostBlock {
   bool used = false;
   Box b{}, b0{}, b1{};
@@ -127,6 +130,19 @@ SlabFit slab_fit(const BlockView* hv, int nblk, int ncta, int rows) {
 }
 size_t slab_smem(const SlabFit& f, int rows) { return (size_t)f.D * rows * (f.So + 2 * f.L) * sizeof(double); }
 
+// Launch shape of the pipelined sweeps for a set of blocks on clusters of C
+// CTAs; ok is false when a plane or such a cluster does not fit.
+struct PipeFit {
+  bool ok = false;
+  int C = 1, threads = 0, variant = 0;
+  PipeShape sh{};
+  size_t smem = 0;
+  double est = 0;  // estimated cycles of the sweeps
+};
+PipeFit pipe_fit(const BlockView* hv, int nblk, int C);
+// The same for the SA equation's sweeps (by the mean flow's order, so for its C).
+PipeFit pipe_sa_fit(const BlockView* hv, int nblk, int C);
+
 // slab_fit of the registered blocks (hv null; cached per setup) or of the
 // nblk host views hv.
 SlabFit slab_fit_for(const BlockView* hv, int nblk, int ncta, int rows);
@@ -170,6 +186,13 @@ struct State {
   size_t smem_slab[5] = {0, 0, 0, 0, 0};
   bool np_slab[5] = {false, false, false, false, false};
   std::map<int, SlabFit> slab_fits;
+  // pipelined sweeps: the registered blocks' launch shape (clusters of pipe.C
+  // CTAs), the one of a drop-in call's own view, and per precision the dynamic
+  // shared memory set so far and whether clusters of 16 are allowed
+  PipeFit pipe, tpipe, pipe_sa, tpipe_sa;
+  size_t smem_pipe_sa = 0;
+  size_t smem_pipe[2][kPipeVariants] = {};
+  bool np_pipe[2][kPipeVariants] = {};
   long spin_limit = kPollBudgetMax;  // polls of each staged-sweep wait (aero_set_poll_budget)
   int stall_plane = -1;              // forward plane whose copies are withheld (aero_inject_sweep_stall)
   bool configured = false;
@@ -239,6 +262,8 @@ struct State {
   bool rhsi_ghosts_zero = false;
   // launch shapes (aero_autotune); none of them changes the arithmetic
   struct Tune {
+    bool sa_pipe = true;  // the same for the SA sweep (false: aero_set_sa_sweep_cluster's)
+    bool pipe = true;   // pipelined sweeps (when they fit); false: the ones aero_set_sweep_cluster selects
     int inv_tile = 64;  // nodes per CTA of the inviscid flux; 0: face-based kernels (-6, -8: FP64 faces for 6, 8 CTAs/SM;
                         // -10: FP64 faces with shared-memory stencils)
     int ew = 256;       // threads per CTA of the element-wise kernels
@@ -411,6 +436,7 @@ size_t view_doubles(long plane) {
 void fill_view(BlockView& v, const Box& b, const Box& b0, const Box& b1, long plane, double* base) {
   v.b = b; v.b0 = b0; v.b1 = b1;
   v.ccb = nullptr;
+  v.pipe = PipeView{};
   v.bstat = nullptr;
   v.live = nullptr;
   v.nx = b.nx(); v.ny = b.ny();
@@ -423,17 +449,30 @@ void fill_view(BlockView& v, const Box& b, const Box& b0, const Box& b1, long pl
 }
 
 // LU-SGS workspace of one view (see BlockView): one device allocation holding
-// poff, rec_f, rec_b, sca, dqs, dq, sa_rec, sa_dq, nat, nbr, pidx, seg, each array
-// starting on a 256-byte boundary (the sweeps' bulk copies and L2 prefetches
+// poff, rec_f, rec_b, sca, dqs, dq, sa_rec, sa_dq, nat, nbr, pidx, seg and the
+// pipelined sweeps' arrays, each array starting on a 256-byte boundary (the sweeps' bulk copies and L2 prefetches
 // of plane chunks need 16-byte aligned starts).
 constexpr size_t kWsAlign = 256;
-constexpr int kWsArrays = 12;
+constexpr int kWsArrays = 17;
+long pipe_plane_max(const Box& b1) { return (long)kPipeSlabs * (b1.nx() + b1.ny() + b1.nz()); }
 size_t ws_round(size_t bytes) { return (bytes + kWsAlign - 1) / kWsAlign * kWsAlign; }
 size_t workspace_bytes(const Box& b1, int H) {
   size_t N1 = (size_t)b1.size();
   return (size_t)(H + 1) * sizeof(long) + N1 * (2 * kRec + kSca + 8 + 5 + kSaRec + 1) * sizeof(double) +
          N1 * sizeof(long) + N1 * 7 * sizeof(int) + (size_t)H * (b1.nz() + 2) * sizeof(int) +
-         (kWsArrays + 1) * kWsAlign;
+         N1 * ((kPipeRec + kPipeSaRec) * sizeof(double) + sizeof(int)) +
+         (size_t)pipe_plane_max(b1) * sizeof(PipePlane) + (kPipeSlabs + 1) * sizeof(int) + (kWsArrays + 1) * kWsAlign;
+}
+// The order of a view's pipelined sweeps for clusters of ncta CTAs: its tables
+// into the view's workspace (k_pipe_index then fills the per-node ones).
+int set_pipe_order(BlockView& v, int ncta) {
+  const PipeTables t = pipe_tables(v.b1, pipe_direction(v.b1, ncta), ncta);
+  v.pipe.dir = t.dir;
+  v.pipe.ce = t.ce;
+  CK(cudaMemcpyAsync(v.pipe.slab, t.slab.data(), t.slab.size() * sizeof(int), cudaMemcpyHostToDevice, g.stream));
+  CK(cudaMemcpyAsync(v.pipe.plane, t.plane.data(), t.plane.size() * sizeof(PipePlane), cudaMemcpyHostToDevice,
+                     g.stream));
+  return AERO_OK;
 }
 int attach_workspace(BlockView& v, void* ws, const std::vector<long>& poff, int pmax) {
   size_t N1 = (size_t)v.b1.size();
@@ -458,10 +497,155 @@ int attach_workspace(BlockView& v, void* ws, const std::vector<long>& poff, int 
   v.pidx = v.nbr + 6 * N1;
   const std::vector<int> seg = plane_segments(v.b1);
   v.seg = (int*)take(seg.size() * sizeof(int));
+  v.pipe.rec = (double*)take(N1 * kPipeRec * sizeof(double));
+  v.pipe.sa_rec = (double*)take(N1 * kPipeSaRec * sizeof(double));
+  v.pipe.at = (int*)take(N1 * sizeof(int));
+  v.pipe.plane = (PipePlane*)take((size_t)pipe_plane_max(v.b1) * sizeof(PipePlane));
+  v.pipe.slab = (int*)take((kPipeSlabs + 1) * sizeof(int));
   CK(cudaMemcpyAsync(v.poff, poff.data(), poff.size() * sizeof(long), cudaMemcpyHostToDevice, g.stream));
   if (!seg.empty())
     CK(cudaMemcpyAsync(v.seg, seg.data(), seg.size() * sizeof(int), cudaMemcpyHostToDevice, g.stream));
   return AERO_OK;
+}
+
+// The kernel of the pipelined sweeps, ready for launches of this shape.
+int prepare_pipe(const PipeFit& pf, int f) {
+  auto kern = pipe_kernel(pf.variant, f);
+  if (pf.smem > g.smem_pipe[f][pf.variant]) {
+    CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pf.smem));
+    g.smem_pipe[f][pf.variant] = pf.smem;
+  }
+  if (pf.C > 8 && !g.np_pipe[f][pf.variant]) {  // 16 CTAs: a non-portable cluster size
+    CK(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    g.np_pipe[f][pf.variant] = true;
+  }
+  return AERO_OK;
+}
+
+PipeFit pipe_fit(const BlockView* hv, int nblk, int C) {
+  PipeFit f;
+  f.C = C;
+  int P = 1, L = 1, H = 1, steps = 1, cuts = 1;
+  for (int m = 0; m < nblk; ++m) {
+    const PipeTables t = pipe_tables(hv[m].b1, pipe_direction(hv[m].b1, C), C);
+    P = std::max(P, t.pmax);
+    L = std::max(L, t.lmax);
+    H = std::max(H, t.hmax);
+    steps = std::max(steps, 2 * (hv[m].b1.nx() + hv[m].b1.ny() + hv[m].b1.nz() - 2));
+    cuts = std::max(cuts, t.ce);
+  }
+  if (P > 1022) return f;  // the neighbour words' index range
+  // one CTA of up to 16 warps per SM or, where the clusters outnumber the SMs,
+  // two of up to 8
+  const bool two = nblk * C > kSms;
+  const int most = two ? 7 : 15;  // compute warps
+  const size_t limit = (size_t)(two ? 113 : 226) * 1024;
+  PipeShape& s = f.sh;
+  s.P = P;
+  s.L = L;
+  s.W = std::min(most, (P + 9) / 10);
+  // up to seven groups while the CTA keeps to 8 warps (200 registers each),
+  // else two within 11 (168 registers)
+  s.NG = s.W <= 3 ? 7 / s.W : (!two && s.W <= 5) ? 2 : 1;
+  s.NST = s.NG + 3;
+  s.D = 8;
+  auto bytes = [&] { return (size_t)PipeSmem(s, kPipeRec, kPipeProd, 5, H).words * sizeof(double); };
+  while (bytes() > limit && s.NST > std::max(2, s.NG)) --s.NST;
+  while (bytes() > limit && s.NG > 1) s.NST = std::max(2, --s.NG);
+  if (bytes() > limit) return f;
+  // more messages on the way while three quarters of that hold them
+  while (s.D < 64 && (s.D *= 2, bytes() <= limit / 4 * 3)) {
+  }
+  if (s.D > 8 && bytes() > limit / 4 * 3) s.D /= 2;
+  f.smem = bytes();
+  f.threads = 32 * (s.W * s.NG + 1);
+  f.variant = two ? 3 : 0;
+  while (kPipeWarps[f.variant] < s.W * s.NG + 1) ++f.variant;
+  // the clusters of this shape that the device holds at a time
+  int active = 0;
+  for (int x = 0; x < 2; ++x) {
+    if (prepare_pipe(f, x) != AERO_OK) {
+      cudaGetLastError();
+      return f;
+    }
+    cudaLaunchConfig_t lc = {};
+    lc.gridDim = dim3((unsigned)(nblk * C));
+    lc.blockDim = dim3((unsigned)f.threads);
+    lc.dynamicSmemBytes = f.smem;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)C;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    lc.attrs = at;
+    lc.numAttrs = 1;
+    if (cudaOccupancyMaxActiveClusters(&active, pipe_kernel(f.variant, x), &lc) != cudaSuccess || active < 1) {
+      cudaGetLastError();
+      return f;
+    }
+  }
+  f.ok = true;
+  // Estimate, from timings of single sweeps, in cycles: a plane's step is bound
+  // by its chain (560) or by a group's way through a plane (1700 and 150 per
+  // warp, 240 past 11 warps, where registers run out) shared out over the
+  // groups; two CTAs on an SM slow each other (1400 and 130 per warp).  A CTA
+  // behind a cut starts about 600 after the one before it.
+  const double step = two ? 1400.0 + 130.0 * s.W
+                          : std::max(560.0, (1700.0 + (s.W > 10 ? 240.0 : 150.0) * s.W) / s.NG);
+  const int passes = (P + 10 * s.W - 1) / (10 * s.W);
+  f.est = ((nblk + active - 1) / active) * (steps * step * passes + 1200.0 * cuts);
+  return f;
+}
+
+PipeFit pipe_sa_fit(const BlockView* hv, int nblk, int C) {
+  PipeFit f;
+  f.C = C;
+  int P = 1, L = 1, H = 1;
+  for (int m = 0; m < nblk; ++m) {
+    const PipeTables t = pipe_tables(hv[m].b1, pipe_direction(hv[m].b1, C), C);
+    P = std::max(P, t.pmax);
+    L = std::max(L, t.lmax);
+    H = std::max(H, t.hmax);
+  }
+  if (P > 1022) return f;
+  PipeShape& s = f.sh;
+  s.P = P;
+  s.L = L;
+  // a node's step is short (a division and a barrier), so its records are read
+  // up to four planes ahead; at most a quarter of the SM's shared memory, which
+  // the mean flow's CTAs beside it need
+  s.W = std::min(15, (P + 31) / 32);
+  s.NG = std::max(1, std::min(4, 15 / s.W));
+  s.NST = s.NG + 3;
+  s.D = 8;
+  auto bytes = [&] { return (size_t)PipeSmem(s, kPipeSaRec, 1, 1, H).words * sizeof(double); };
+  while (bytes() > 56 * 1024 && s.NST > std::max(2, s.NG)) --s.NST;
+  if (bytes() > 200 * 1024) return f;
+  while (s.D < 64 && (s.D *= 2, bytes() <= 56 * 1024)) {
+  }
+  if (s.D > 8 && bytes() > 56 * 1024) s.D /= 2;
+  f.smem = bytes();
+  f.threads = 32 * (s.W * s.NG + 1);
+  if (f.smem > g.smem_pipe_sa) {
+    if (cudaFuncSetAttribute(k_pipe_sa_sweep, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)f.smem) != cudaSuccess ||
+        cudaFuncSetAttribute(k_pipe_sa_sweep, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+      cudaGetLastError();
+      return f;
+    }
+    g.smem_pipe_sa = f.smem;
+  }
+  f.ok = true;
+  return f;
+}
+
+// The pipelined sweeps' cluster size by rule: the smallest estimate of pipe_fit.
+PipeFit pipe_choose(const BlockView* hv, int nblk) {
+  PipeFit best;
+  for (int C : {1, 2, 4, 8, 16}) {
+    const PipeFit f = pipe_fit(hv, nblk, C);
+    if (f.ok && (!best.ok || f.est < best.est)) best = f;
+  }
+  return best;
 }
 
 int ensure_staging(size_t doubles) {
@@ -692,8 +876,13 @@ int launch_dt_minmax(const BlockView* views, int m, double* d_out2) {
 // (the library's stream when null).  A steady iteration runs it on its own
 // stream beside the flux and time-step kernels.
 int launch_implicit_blocks(const BlockView* views, int nblk, long maxExt, long maxN1, const CaseConsts& cc,
-                           cudaStream_t st = nullptr) {
+                           cudaStream_t st, const PipeFit& pf) {
   if (!st) st = g.stream;
+  if (g.tune.pipe && pf.ok) {
+    PROF_ON(P_LUSGS_MATS, st, (k_pipe_recs<<<dim3(cdiv(maxN1, 128), nblk), 128, 0, st>>>(views, cc)));
+    CKL();
+    return AERO_OK;
+  }
   const int f = g.mixed ? 1 : 0;
   PROF_ON(P_LUSGS_RADII, st, (k_lusgs_radii<<<dim3(cdiv(maxExt, g.tune.ew), nblk), g.tune.ew, 0, st>>>(views)));
   CKL();
@@ -742,14 +931,31 @@ int prepare_slab(K kern, int k, size_t smem, int cl) {
 }
 
 int launch_implicit(const BlockView* views, int nblk, long maxExt, long maxN1, int pmax, int hmax,
-                    const CaseConsts& cc, cudaEvent_t after_prep = nullptr, bool with_blocks = true,
+                    const CaseConsts& cc, const PipeFit& pf, cudaEvent_t after_prep = nullptr, bool with_blocks = true,
                     const BlockView* sweep_views = nullptr, const BlockView* host_views = nullptr) {
+  if (g.tune.pipe && pf.ok) {
+    int rc;
+    if (with_blocks && (rc = launch_implicit_blocks(views, nblk, maxExt, maxN1, cc, nullptr, pf))) return rc;
+    PROF(P_LUSGS_SCA, (k_pipe_sca<<<dim3(cdiv(maxN1, 128), nblk), 128, 0, g.stream>>>(views, cc)));
+    CKL();
+    if (after_prep) CK(cudaEventRecord(after_prep, g.stream));
+    const int f = g.mixed ? 1 : 0;
+    if ((rc = prepare_pipe(pf, f))) return rc;
+    cudaError_t le = cudaSuccess;
+    PROF(P_LUSGS_SWEEP,
+         (le = launch_clusters(pipe_kernel(pf.variant, f), nblk, pf.C, pf.threads, pf.smem, g.stream,
+                               sweep_views ? sweep_views : views, cc, pf.sh, g.d_status, g.spin_limit, g.stall_plane)));
+    CK(le);
+    PROF(P_LUSGS_UPDATE, (k_pipe_update<<<dim3(cdiv(maxN1, 256), nblk), 256, 0, g.stream>>>(views)));
+    CKL();
+    return AERO_OK;
+  }
   const BlockView* sv = sweep_views ? sweep_views : views;
   // mixed precision stores the off-diagonal blocks in FP32 (products and sums
   // stay FP64); f selects that variant of every kernel that touches them
   const int f = g.mixed ? 1 : 0;
   int rc;
-  if (with_blocks && (rc = launch_implicit_blocks(views, nblk, maxExt, maxN1, cc))) return rc;
+  if (with_blocks && (rc = launch_implicit_blocks(views, nblk, maxExt, maxN1, cc, nullptr, pf))) return rc;
   PROF(P_LUSGS_PREP, (k_lusgs_prep<<<dim3(cdiv(maxExt, g.tune.ew), nblk), g.tune.ew, 0, g.stream>>>(views, cc)));
   CKL();
   if (after_prep) CK(cudaEventRecord(after_prep, g.stream));
@@ -883,6 +1089,11 @@ int launch_implicit(const BlockView* views, int nblk, long maxExt, long maxN1, i
   return AERO_OK;
 }
 
+int launch_pipe_index(const BlockView* views, int nblk, long maxN1) {
+  PROF(P_INDEX, (k_pipe_index<<<dim3(cdiv(maxN1, 256), nblk), 256, 0, g.stream>>>(views)));
+  CKL();
+  return AERO_OK;
+}
 int launch_index(const BlockView* views, int nblk, long maxN1) {
   PROF(P_INDEX, (k_plane_index<<<dim3(cdiv(maxN1, 256), nblk), 256, 0, g.stream>>>(views)));
   CKL();
@@ -895,7 +1106,7 @@ int launch_index(const BlockView* views, int nblk, long maxN1) {
 // pri_v, amu, vor, dudx and the metrics), 2 the records and the sweeps (the
 // records also read dt); 3 both.
 int launch_sa(const BlockView* views, int nblk, long maxN, long maxN1, int pmax, const CaseConsts& cc,
-              cudaStream_t st = nullptr, const BlockView* host_views = nullptr, int parts = 3) {
+              const PipeFit& pf, cudaStream_t st = nullptr, const BlockView* host_views = nullptr, int parts = 3) {
   if (!st) st = g.stream;
   if (parts & 1) {
     PROF_ON(P_FILL, st, (k_sa_length<<<dim3(cdiv(maxN, 256), nblk), 256, 0, st>>>(views, cc)));
@@ -907,6 +1118,15 @@ int launch_sa(const BlockView* views, int nblk, long maxN, long maxN1, int pmax,
     CKL();
   }
   if (!(parts & 2)) return AERO_OK;
+  if (g.tune.sa_pipe && pf.ok) {
+    PROF_ON(P_SA_RECS, st, (k_pipe_sa_recs<<<dim3(cdiv(maxN1, 128), nblk), 128, 0, st>>>(views, cc)));
+    CKL();
+    cudaError_t le = cudaSuccess;
+    PROF_ON(P_SA_SWEEP, st, (le = launch_clusters(k_pipe_sa_sweep, nblk, pf.C, pf.threads, pf.smem, st, views, cc, pf.sh,
+                                                  g.d_status, kPipePolls, -1)));
+    CK(le);
+    return AERO_OK;
+  }
   PROF_ON(P_SA_RECS, st, (k_sa_recs<<<dim3(cdiv(maxN1, 256), nblk), 256, 0, st>>>(views, cc)));
   CKL();
   SlabFit sf;
@@ -927,6 +1147,54 @@ int launch_sa(const BlockView* views, int nblk, long maxN, long maxN1, int pmax,
   PROF_ON(P_SA_SWEEP, st, ((threads <= 768 ? k_sa_sweep_768 : k_sa_sweep)<<<nblk, threads, smem, st>>>(views)));
   CKL();
   return AERO_OK;
+}
+
+void graph_release();
+
+// The registered blocks' views to the device: in block order, and with the
+// longest hyperplane chains first for the LU-SGS sweeps (when a batch's sweep
+// CTAs outnumber the SMs, the blocks whose sweeps take longest are the first
+// to be given SMs).
+int upload_views() {
+  const size_t bytes = g.views.size() * sizeof(BlockView);
+  CK(cudaMemcpyAsync(g.d_blocks, g.views.data(), bytes, cudaMemcpyHostToDevice, g.stream));
+  std::vector<BlockView> chain(g.views);
+  std::stable_sort(chain.begin(), chain.end(),
+                   [](const BlockView& a, const BlockView& b) { return a.nplanes > b.nplanes; });
+  CK(cudaMemcpyAsync(g.d_blocks_chain, chain.data(), bytes, cudaMemcpyHostToDevice, g.stream));
+  return AERO_OK;
+}
+
+// The registered blocks' pipelined sweeps on clusters of C CTAs (1, 2, 4, 8
+// or 16): the order's tables again, and the views that hold them.  *fits is
+// false (and nothing changes) when a plane or such a cluster does not fit.
+int set_pipe_cluster(int C, bool* fits) {
+  const int nb = (int)g.blocks.size();
+  const PipeFit f = pipe_fit(g.views.data(), nb, C);
+  *fits = f.ok;
+  if (!f.ok) return AERO_OK;
+  g.pipe = f;
+  g.pipe_sa = pipe_sa_fit(g.views.data(), nb, C);
+  for (int m = 0; m < nb; ++m) {
+    int rc = set_pipe_order(g.views[m], C);
+    if (rc) return rc;
+  }
+  int rc = upload_views();
+  if (rc) return rc;
+  graph_release();
+  return launch_pipe_index(g.d_blocks, nb, g.max_b1);
+}
+
+// The sweeps' orders of a drop-in call's own view.
+int transient_order(BlockTarget& t, long N1) {
+  g.tpipe = pipe_choose(&t.view, 1);
+  g.tpipe_sa = pipe_sa_fit(&t.view, 1, g.tpipe.C);
+  int rc = set_pipe_order(t.view, g.tpipe.C);
+  if (rc) return rc;
+  CK(cudaMemcpyAsync(g.d_tview, &t.view, sizeof(BlockView), cudaMemcpyHostToDevice, g.stream));
+  if ((rc = launch_pipe_index(t.d_view, 1, N1))) return rc;
+  const bool all = g.tune.pipe && g.tpipe.ok && g.tune.sa_pipe && g.tpipe_sa.ok;
+  return all ? AERO_OK : launch_index(t.d_view, 1, N1);
 }
 
 bool viscous_on() { return g.cc.solver == IFLAG_NSSOLVER; }
@@ -1030,7 +1298,7 @@ int do_iteration_crank() {
   }
   PROF(P_CRANK, (k_update_q0<<<dim3(cdiv(g.max_b0, 256), nb), 256, 0, g.stream>>>(g.d_blocks)));
   CKL();
-  if (sa_on() && (rc = launch_sa(g.d_blocks, nb, g.max_box, g.max_b1, g.pmax_all, g.cc))) return rc;
+  if (sa_on() && (rc = launch_sa(g.d_blocks, nb, g.max_box, g.max_b1, g.pmax_all, g.cc, g.pipe_sa))) return rc;
   if ((rc = do_physical_bc())) return rc;
   if ((rc = do_halo())) return rc;
   if ((rc = do_average1())) return rc;
@@ -1072,7 +1340,7 @@ int do_iteration(bool want_dt_minmax, bool resid_beside = false) {
   // both: nothing before the sweeps writes what they read or reads what they
   // write
   CK(cudaStreamWaitEvent(g.stream3, g.ev_fork2, 0));
-  if ((rc = launch_implicit_blocks(g.d_blocks, nb, g.max_ext, g.max_b1, g.cc, g.stream3))) return rc;
+  if ((rc = launch_implicit_blocks(g.d_blocks, nb, g.max_ext, g.max_b1, g.cc, g.stream3, g.pipe))) return rc;
   CK(cudaEventRecord(g.ev_join3, g.stream3));
   // viscous part a, then find_dt (it reads the viscosity part a forms);
   // sa_model runs on a fourth stream: it reads pri_v, amu, dudx, vor, dt and
@@ -1085,20 +1353,20 @@ int do_iteration(bool want_dt_minmax, bool resid_beside = false) {
   if (sa) {
     CK(cudaEventRecord(g.ev_fork, g.stream));
     CK(cudaStreamWaitEvent(g.stream4, g.ev_fork, 0));
-    if ((rc = launch_sa(g.d_blocks, nb, g.max_box, g.max_b1, g.pmax_all, g.cc, g.stream4, nullptr, 1))) return rc;
+    if ((rc = launch_sa(g.d_blocks, nb, g.max_box, g.max_b1, g.pmax_all, g.cc, g.pipe_sa, g.stream4, nullptr, 1))) return rc;
   }
   if ((rc = launch_find_dt(g.d_blocks, nb, g.max_box, g.cc))) return rc;
   if (want_dt_minmax && (rc = launch_dt_minmax(g.d_blocks, nb - 1, g.d_out + 7))) return rc;
   if (sa) {
     CK(cudaEventRecord(g.ev_dt, g.stream));
     CK(cudaStreamWaitEvent(g.stream4, g.ev_dt, 0));
-    if ((rc = launch_sa(g.d_blocks, nb, g.max_box, g.max_b1, g.pmax_all, g.cc, g.stream4, nullptr, 2))) return rc;
+    if ((rc = launch_sa(g.d_blocks, nb, g.max_box, g.max_b1, g.pmax_all, g.cc, g.pipe_sa, g.stream4, nullptr, 2))) return rc;
     CK(cudaEventRecord(g.ev_join, g.stream4));
   }
   if (viscous_on() && (rc = launch_viscous_b(g.d_blocks, nb, g.max_b0, g.cc))) return rc;
   CK(cudaStreamWaitEvent(g.stream, g.ev_join2, 0));
   CK(cudaStreamWaitEvent(g.stream, g.ev_join3, 0));
-  if ((rc = launch_implicit(g.d_blocks, nb, g.max_ext, g.max_b1, g.pmax_all, g.hmax_all, g.cc,
+  if ((rc = launch_implicit(g.d_blocks, nb, g.max_ext, g.max_b1, g.pmax_all, g.hmax_all, g.cc, g.pipe,
                             resid_beside ? g.ev_prep : nullptr, false, g.d_blocks_chain)))
     return rc;
   if (resid_beside) {
@@ -1204,7 +1472,14 @@ const char* aero_last_error(void) { return g.err.c_str(); }
 int aero_init(int device) {
   if (g.inited) return AERO_OK;
   CK(cudaSetDevice(device));
-  for (int f = 0; f < 2; ++f) g.smem_staged[f] = 0;
+  g.smem_pipe_sa = 0;
+  for (int f = 0; f < 2; ++f) {
+    g.smem_staged[f] = 0;
+    for (int v = 0; v < kPipeVariants; ++v) {
+      g.smem_pipe[f][v] = 0;
+      g.np_pipe[f][v] = false;
+    }
+  }
   for (int f = 0; f < 6; ++f) {
     g.smem_bulk[f] = 0;
     g.np_cluster[f] = false;
@@ -1314,6 +1589,8 @@ int aero_finalize(void) {
   g.tuning = State{}.tuning;
   return AERO_OK;
 }
+
+void set_tuning_text(void);
 
 int aero_set_block_params(int m, const double* params) {
   int rc = need_init();
@@ -1434,13 +1711,15 @@ bool slab_cluster16_fits(int rows) {
 
 const char* exchange_name(int x) { return x == 3 ? "shared2" : x == 2 ? "slab" : x == 1 ? "shared" : "l2"; }
 
-void set_tuning_text() {
+void set_tuning_text(void) {
   char buf[280];
+  const bool piped = g.tune.pipe && g.setup && g.pipe.ok;
   std::snprintf(buf, sizeof buf,
                 "inviscid_tile=%d elementwise_threads=%d viscous_threads=%d mats_threads=%d sweep_stages<=%d "
                 "sweep_cluster=%d sweep_exchange=%s sa_sweep_cluster=%d register_bound=%d sweep_prefetch=%d",
-                g.tune.inv_tile, g.tune.ew, g.tune.visc, g.tune.mats, g.tune.nst_max, std::max(1, g.tune.sweep_cl),
-                exchange_name(g.tune.sweep_x), std::max(1, g.tune.sa_cl), g.tune.bound, g.tune.sweep_pf);
+                g.tune.inv_tile, g.tune.ew, g.tune.visc, g.tune.mats, g.tune.nst_max,
+                piped ? g.pipe.C : std::max(1, g.tune.sweep_cl), piped ? "pipelined" : exchange_name(g.tune.sweep_x),
+                g.tune.sa_pipe && g.setup && g.pipe_sa.ok ? g.pipe_sa.C : std::max(1, g.tune.sa_cl), g.tune.bound, g.tune.sweep_pf);
   g.tuning = buf;
 }
 
@@ -1492,18 +1771,25 @@ int aero_autotune(int iters) {
   // the sweep's cluster size and exchange are one knob (value 4 * ctas +
   // exchange), since the exchanges are only eligible for some sizes
   int sweep_mode = 4 * g.tune.sweep_cl + g.tune.sweep_x;
+  // the pipelined sweeps' CTAs per block (the mode above where they are off)
+  int pipe_c = g.pipe.C;
+  const bool piped = g.tune.pipe && g.pipe.ok;
   struct Knob { int* v; std::vector<int> cand; };
   std::vector<Knob> knobs = {{&g.tune.inv_tile, {0, -6, -8, -10, 32, 64, 128}}, {&g.tune.ew, {128, 256, 512}},
                              {&g.tune.visc, {64, 128, 256}}, {&g.tune.mats, {64, 128, 256}},
-                             {&g.tune.nst_max, {2, 3, 4}},
-                             {&sweep_mode, {0, 8, 16, 32, 9, 17, 33, 10, 18, 34, 11, 19, 35}},
-                             {&g.tune.bound, {0, 1}}, {&g.tune.sweep_pf, {2, 3, 4}}};
-  for (Knob& k : knobs)
-    if (k.v == &sweep_mode) {
-      if (bulk_cluster16_fits()) k.cand.push_back(65);   // 16 CTAs, bulk exchange
-      if (slab_cluster16_fits(5)) k.cand.push_back(66);  // 16 CTAs, slabs
-    }
-  if (sa_on()) {
+                             {&g.tune.bound, {0, 1}}};
+  if (piped) {
+    knobs.push_back({&pipe_c, {}});
+    for (int C : {1, 2, 4, 8, 16})
+      if (pipe_fit(g.views.data(), nb, C).ok) knobs.back().cand.push_back(C);
+  } else {
+    knobs.push_back({&g.tune.nst_max, {2, 3, 4}});
+    knobs.push_back({&sweep_mode, {0, 8, 16, 32, 9, 17, 33, 10, 18, 34, 11, 19, 35}});
+    if (bulk_cluster16_fits()) knobs.back().cand.push_back(65);   // 16 CTAs, bulk exchange
+    if (slab_cluster16_fits(5)) knobs.back().cand.push_back(66);  // 16 CTAs, slabs
+    knobs.push_back({&g.tune.sweep_pf, {2, 3, 4}});
+  }
+  if (sa_on() && !(g.tune.sa_pipe && g.pipe_sa.ok)) {
     knobs.push_back({&g.tune.sa_cl, {0, 2, 4, 8}});
     if (slab_cluster16_fits(1)) knobs.back().cand.push_back(16);
   }
@@ -1514,6 +1800,8 @@ int aero_autotune(int iters) {
       *k.v = c;
       g.tune.sweep_cl = sweep_mode / 4;
       g.tune.sweep_x = sweep_mode % 4;
+      bool fits = true;
+      if (pipe_c != g.pipe.C && ((rc = set_pipe_cluster(pipe_c, &fits)) || !fits)) break;
       double ms = 0;
       if ((rc = time_steps(ms))) break;
       if (ms < best_ms) { best_ms = ms; best = c; }
@@ -1521,6 +1809,8 @@ int aero_autotune(int iters) {
     *k.v = best;
     g.tune.sweep_cl = sweep_mode / 4;
     g.tune.sweep_x = sweep_mode % 4;
+    bool fits = true;
+    if (!rc && pipe_c != g.pipe.C) rc = set_pipe_cluster(pipe_c, &fits);
     if (rc) break;
   }
   cudaEventDestroy(a);
@@ -1596,6 +1886,7 @@ int aero_set_sweep_cluster(int ctas) {
     return fail(AERO_ERR_ARG, "a cluster of 16 sweep CTAs does not fit this device or these blocks "
                               "(16 CTAs take the bulk or the slab exchange only)");
   g.tune.sweep_cl = ctas == 1 ? 0 : ctas;
+  g.tune.pipe = false;
   graph_release();
   set_tuning_text();
   return AERO_OK;
@@ -1629,6 +1920,7 @@ int aero_set_sa_sweep_cluster(int ctas) {
   if (ctas == 16 && !slab_cluster16_fits(1))
     return fail(AERO_ERR_ARG, "a cluster of 16 SA sweep CTAs does not fit this device or these blocks");
   g.tune.sa_cl = ctas == 1 ? 0 : ctas;
+  g.tune.sa_pipe = false;
   graph_release();
   set_tuning_text();
   return AERO_OK;
@@ -1840,6 +2132,10 @@ int aero_finish_setup(void) {
     g.pmax_all = std::max(g.pmax_all, pmax);
     g.hmax_all = std::max(g.hmax_all, (int)poff.size() - 1);
   }
+  g.pipe = pipe_choose(g.views.data(), nb);
+  g.pipe_sa = pipe_sa_fit(g.views.data(), nb, g.pipe.C);
+  for (int m = 0; m < nb; ++m)
+    if ((rc = set_pipe_order(g.views[m], g.pipe.C))) return rc;
   // per-block case constants of a batch (aero_set_block_params)
   bool any_own = false;
   for (auto& H : g.blocks) any_own = any_own || H.own_params;
@@ -1865,17 +2161,8 @@ int aero_finish_setup(void) {
     g.views[m].live = g.d_live + m;
   }
   CK(cudaMalloc(&g.d_blocks, nb * sizeof(BlockView)));
-  CK(cudaMemcpyAsync(g.d_blocks, g.views.data(), nb * sizeof(BlockView), cudaMemcpyHostToDevice, g.stream));
-  // the same views with the longest hyperplane chains first, for the LU-SGS
-  // sweeps: when a batch's sweep CTAs outnumber the SMs, the blocks whose
-  // sweeps take longest are the first to be given SMs
-  {
-    std::vector<BlockView> chain(g.views);
-    std::stable_sort(chain.begin(), chain.end(),
-                     [](const BlockView& a, const BlockView& b) { return a.nplanes > b.nplanes; });
-    CK(cudaMalloc(&g.d_blocks_chain, nb * sizeof(BlockView)));
-    CK(cudaMemcpyAsync(g.d_blocks_chain, chain.data(), nb * sizeof(BlockView), cudaMemcpyHostToDevice, g.stream));
-  }
+  CK(cudaMalloc(&g.d_blocks_chain, nb * sizeof(BlockView)));
+  if ((rc = upload_views())) return rc;
   // tables
   CK(cudaMalloc(&g.d_bc_ops, std::max<size_t>(1, topo.bc_ops.size()) * sizeof(BcOp)));
   if (!topo.bc_ops.empty())
@@ -1918,6 +2205,8 @@ int aero_finish_setup(void) {
   if (g.navg_src) CK(cudaMemcpyAsync(g.d_avg_src, topo.avg_src.data(), g.navg_src * sizeof(AvgSrc), cudaMemcpyHostToDevice, g.stream));
   if (g.navg_dst) CK(cudaMemcpyAsync(g.d_avg_dst, topo.avg_dst.data(), g.navg_dst * sizeof(AvgDst), cudaMemcpyHostToDevice, g.stream));
   if ((rc = launch_index(g.d_blocks, nb, g.max_b1))) return rc;
+  if ((rc = launch_pipe_index(g.d_blocks, nb, g.max_b1))) return rc;
+  if ((rc = launch_pipe_index(g.d_blocks, nb, g.max_b1))) return rc;
   g.resid_ctas = (int)cdiv(g.max_b1, 256);
   CK(cudaMalloc(&g.d_part, (size_t)g.resid_ctas * nb * 6 * sizeof(double)));
   CK(cudaMalloc(&g.d_resid_blocks, (size_t)nb * 7 * sizeof(double)));
@@ -1972,6 +2261,7 @@ int aero_finish_setup(void) {
   }
   CK(cudaStreamSynchronize(g.stream));
   g.setup = true;
+  set_tuning_text();
   return AERO_OK;
 }
 
@@ -2273,9 +2563,9 @@ int aero_implicit1st(double* q, const double* dt, const double* pri_v, double* r
   CaseConsts cc = consts_with(*gamma, g.cc.cv, g.cc.re);
   cc.cfl = *cfl;
   Box e = grown_box(b, b1);
-  if (!t.resident && (rc = launch_index(t.d_view, 1, b1.size()))) return rc;
-  if ((rc = launch_implicit(t.d_view, 1, e.size(), b1.size(), t.view.pmax, t.view.nplanes, cc, nullptr, true,
-                            nullptr, &t.view)))
+  if (!t.resident && (rc = transient_order(t, b1.size()))) return rc;
+  if ((rc = launch_implicit(t.d_view, 1, e.size(), b1.size(), t.view.pmax, t.view.nplanes, cc,
+                            t.resident ? g.pipe : g.tpipe, nullptr, true, nullptr, &t.view)))
     return rc;
   return finish(t, args);
 }
@@ -2499,8 +2789,10 @@ int aero_sa_model(double* nut, double* sa_rhs, const double* dt, const double* p
   if ((rc = resolve(b, b0, b1, args, t))) return rc;
   CaseConsts cc = consts_with(g.cc.gamma, g.cc.cv, *re);
   cc.cfl = *cfl;
-  if (!t.resident && (rc = launch_index(t.d_view, 1, b1.size()))) return rc;
-  if ((rc = launch_sa(t.d_view, 1, b.size(), b1.size(), t.view.pmax, cc, nullptr, &t.view))) return rc;
+  if (!t.resident && (rc = transient_order(t, b1.size()))) return rc;
+  if ((rc = launch_sa(t.d_view, 1, b.size(), b1.size(), t.view.pmax, cc, t.resident ? g.pipe_sa : g.tpipe_sa, nullptr,
+                      &t.view)))
+    return rc;
   return finish(t, args);
 }
 

@@ -337,4 +337,58 @@ std::string build_topology(const std::vector<TopoBlock>& blocks, int buffer_leng
   return std::string();
 }
 
+// --------------------------------------------- order of the pipelined sweeps
+namespace {
+// nodes of every hyperplane of an n0 x n1 x n2 box
+std::vector<int> plane_counts(const int n[3]) {
+  std::vector<int> cnt(std::max(0, n[0] + n[1] + n[2] - 2), 0);
+  for (int c = 0; c < n[2]; ++c)
+    for (int s = 0; s <= n[0] + n[1] - 2; ++s)
+      cnt[s + c] += std::min(s, n[1] - 1) - std::max(0, s - (n[0] - 1)) + 1;
+  return cnt;
+}
+}  // namespace
+
+PipeTables pipe_tables(const Box& b1, int dir, int ce) {
+  PipeTables t;
+  const int n1[3] = {b1.nx(), b1.ny(), b1.nz()};
+  t.dir = dir;
+  t.ce = std::max(1, std::min(ce, n1[dir]));
+  std::vector<int> cnt;
+  int last = -1, pos = 0;
+  for (int r = 0; r < t.ce; ++r) {
+    int n[3] = {n1[0], n1[1], n1[2]};
+    n[dir] = (int)((long)(r + 1) * n1[dir] / t.ce) - (int)((long)r * n1[dir] / t.ce);
+    if (n[dir] != last) cnt = plane_counts(n);
+    last = n[dir];
+    t.slab.push_back((int)t.plane.size());
+    t.hmax = std::max(t.hmax, (int)cnt.size());
+    for (int c : cnt) {
+      t.plane.push_back(PipePlane{pos, c});
+      pos += c;
+      t.pmax = std::max(t.pmax, c);
+    }
+  }
+  t.slab.push_back((int)t.plane.size());
+  const int u = dir == 0 ? 1 : 0, v = dir == 2 ? 1 : 2;
+  t.lmax = std::min(n1[u], n1[v]);
+  return t;
+}
+
+int pipe_direction(const Box& b1, int ncta) {
+  int best = 0, best_p = 0;
+  for (int dir = 2; dir >= 0; --dir) {
+    int n[3] = {b1.nx(), b1.ny(), b1.nz()};
+    const int ce = std::max(1, std::min(ncta, n[dir]));
+    n[dir] = (n[dir] + ce - 1) / ce;
+    int p = 0;
+    for (int c : plane_counts(n)) p = std::max(p, c);
+    if (dir == 2 || p < best_p) {
+      best = dir;
+      best_p = p;
+    }
+  }
+  return best;
+}
+
 }  // namespace aero

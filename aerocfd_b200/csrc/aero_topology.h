@@ -42,4 +42,22 @@ std::string build_topology(const std::vector<TopoBlock>& blocks, int buffer_leng
 // level within its block (build_topology calls it).
 void bc_levels(Topology& out);
 
+// Host tables of the pipelined sweeps' order (PipeView) of one updated box cut
+// along `dir` into `ce` slabs: the slabs' first planes, every plane's first
+// position and node count; pmax the largest plane, lmax the largest message across a cut (nodes), hmax the most planes of a slab.
+struct PipeTables {
+  int dir = 0, ce = 1, pmax = 0, lmax = 0, hmax = 0;
+  std::vector<int> slab;
+  std::vector<PipePlane> plane;
+};
+PipeTables pipe_tables(const Box& b1, int dir, int ce);
+
+// Slabs of a block at most.
+constexpr int kPipeSlabs = 16;
+// The direction to cut for clusters of ncta CTAs: the one whose slabs have the
+// smallest largest plane (a cut of a short direction leaves every slab most of
+// the block's planes, so that the CTAs all work most of the time; a cut of a
+// long one leaves few and wide ones).
+int pipe_direction(const Box& b1, int ncta);
+
 }  // namespace aero
