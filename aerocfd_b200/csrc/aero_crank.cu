@@ -9,6 +9,7 @@
 // (natural order, zero outside the updated box).  q0 holds the two earlier
 // time levels: component plane (l+1) + 2*(c-1) is q0(l, c), l = -1, 0.
 #include <cmath>
+#include <type_traits>
 
 #include "aero_device.cuh"
 #include "aero_kernels.h"
@@ -81,7 +82,151 @@ __global__ void k_crank_rhs(const BlockView* __restrict__ blocks) {
   }
 }
 
-// One direction's recurrences: thread = one line of the updated box along
+// One direction's recurrences with the lines in shared memory: a CTA takes
+// `lpc` lines of direction d (0: i, 1: j, 2: k).  All its threads form what the
+// recurrences read of every node (the neighbour term's factors, the radius,
+// the pivot), one warp then walks the lines, a lane per line, and all threads
+// store the result.  Walking the lines through global memory, as
+// k_crank_sweep does, takes a memory latency per node; from shared memory a node
+// costs its chain of about ten dependent FP64 operations (97 x 49 x 5 channel: i
+// lines 555 -> 56 us, j lines 200 -> 31, k lines 15 -> 13).  The i lines form
+// the dual-time rhs on the way (:62-87), the last direction adds dq/inv_j to q
+// (:455-462).  The forward recurrence of the k lines starts at ks1+1 and the
+// backward one at ke1-1 (:352, :398), as in the reference; along i and j they
+// cover the whole line.  A neighbour outside the updated box has dq = 0.
+namespace {
+enum LineWord { LW_CU = 0, LW_X, LW_Y, LW_Z, LW_Q2, LW_U, LW_V, LW_W, LW_H, LW_R, LW_HDV, LW_DIV, LW_DQ, LW_NUM = LW_DQ + 5 };
+}
+__global__ void __launch_bounds__(256) k_crank_lines(const BlockView* __restrict__ blocks, int d, int lpc, double gamma,
+                                                     int last) {
+  extern __shared__ double sm[];
+  const BlockView& B = blocks[blockIdx.y];
+  if (B.retired()) return;
+  const Box& b1 = B.b1;
+  const int n1[3] = {b1.nx(), b1.ny(), b1.nz()};
+  const int lo[3] = {b1.is, b1.js, b1.ks};
+  const int u1 = d == 0 ? 1 : 0, u2 = d == 2 ? 1 : 2;  // the two other directions
+  const int len = n1[d], lines = n1[u1] * n1[u2];
+  const int line0 = blockIdx.x * lpc;
+  if (line0 >= lines) return;
+  const int nl = min(lpc, lines - line0);
+  const long st = d == 0 ? 1 : (d == 1 ? (long)B.nx : (long)B.nx * B.ny);
+  const int cb = 3 * d + 1;
+  const double inv1 = 1.0 + kAlph;
+  // word w of node x (-1 .. len) of line l; the row stride is odd, so threads on
+  // neighbouring nodes of one line write different banks
+  const int row = LW_NUM * lpc + 1 - (LW_NUM * lpc & 1);
+  auto at = [&](int x, int w, int l) -> double& { return sm[(x + 1) * row + w * lpc + l]; };
+  auto node = [&](int l, int x) {
+    int ijk[3];
+    ijk[u1] = lo[u1] + (line0 + l) % n1[u1];
+    ijk[u2] = lo[u2] + (line0 + l) / n1[u1];
+    ijk[d] = lo[d] + x;
+    return B.at(ijk[0], ijk[1], ijk[2]);
+  };
+  // threads run along the lines for i, across them (along i) otherwise
+  for (int t = threadIdx.x; t < (len + 2) * nl; t += blockDim.x) {
+    const int l = d == 0 ? t / (len + 2) : t % nl, x = (d == 0 ? t % (len + 2) : t / nl) - 1;
+    const long n = node(l, x);
+    const double u = B.v(F_PRI, 2, n), v = B.v(F_PRI, 3, n), w = B.v(F_PRI, 4, n), c = B.v(F_PRI, 7, n);
+    const double x0 = B.v(F_DXIDX, cb, n), y0 = B.v(F_DXIDX, cb + 1, n), z0 = B.v(F_DXIDX, cb + 2, n);
+    const double q2 = 0.5 * (p2(u) + p2(v) + p2(w));
+    const double r = crank_rou(B, cb, n);
+    at(x, LW_CU, l) = x0 * u + y0 * v + z0 * w;
+    at(x, LW_X, l) = x0;
+    at(x, LW_Y, l) = y0;
+    at(x, LW_Z, l) = z0;
+    at(x, LW_Q2, l) = q2;
+    at(x, LW_U, l) = u;
+    at(x, LW_V, l) = v;
+    at(x, LW_W, l) = w;
+    at(x, LW_H, l) = p2(c) / (gamma - 1.0) + q2;
+    at(x, LW_R, l) = r;
+    const bool inside = x >= 0 && x < len;
+    const double dt = inside ? B.s(F_DT, n) : 0.0;
+    const double dtsub = dt / inv1;
+    at(x, LW_HDV, l) = 0.5 * dtsub;
+    at(x, LW_DIV, l) = 1.0 / (1.0 + dtsub * r);
+    const double alph_i = 1.0 / (1.0 + kAlph), ij = d == 0 && inside ? B.s(F_INVJ, n) : 0.0;
+#pragma unroll
+    for (int k = 1; k <= 5; ++k) {
+      double base = 0.0;
+      if (inside && d == 0) {
+        const double rhs = B.v(F_RHSI, k, n) + B.v(F_RHSV, k, n);
+        base = alph_i * (rhs * dt - ((1.0 + kAlph) * B.v(F_Q, k, n) - (1.0 + 2.0 * kAlph) * q0v(B, 0, k, n) +
+                                     kAlph * q0v(B, -1, k, n)) * ij);
+        B.v(F_RHS, k, n) = base;
+      } else if (inside) {
+        base = dqv(B, k, n);
+      }
+      at(x, LW_DQ + k - 1, l) = base;
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    const int l = min((int)threadIdx.x, nl - 1);  // further lanes repeat the last line
+    auto walk = [&](auto forward, int from, int to, int by) {
+      constexpr bool F = decltype(forward)::value;
+      if (F ? from >= to : from <= to) return;
+      // the neighbour's dq, and its factors one node ahead of their use
+      double s[5], f[10], hdv, div, base[5];
+#pragma unroll
+      for (int k = 0; k < 5; ++k) s[k] = at(from - by, LW_DQ + k, l);
+      auto fetch = [&](int x) {
+#pragma unroll
+        for (int k = 0; k < 10; ++k) f[k] = at(x - by, k, l);
+        hdv = at(x, LW_HDV, l);
+        div = at(x, LW_DIV, l);
+#pragma unroll
+        for (int k = 0; k < 5; ++k) base[k] = at(x, LW_DQ + k, l);
+      };
+      fetch(from);
+      for (int x = from; x != to; x += by) {
+        const double b1 = hdv * (-(f[LW_CU] * s[0]) + f[LW_X] * s[1] + f[LW_Y] * s[2] + f[LW_Z] * s[3]);
+        const double b2 = hdv * (f[LW_Q2] * s[0] - f[LW_U] * s[1] - f[LW_V] * s[2] - f[LW_W] * s[3] + s[4]) * (gamma - 1.0);
+        const double b3 = F ? hdv * (f[LW_CU] + f[LW_R]) : hdv * (f[LW_CU] - f[LW_R]);
+        double a[5];
+        a[0] = b1 + b3 * s[0];
+        a[1] = b1 * f[LW_U] + b2 * f[LW_X] + b3 * s[1];
+        a[2] = b1 * f[LW_V] + b2 * f[LW_Y] + b3 * s[2];
+        a[3] = b1 * f[LW_W] + b2 * f[LW_Z] + b3 * s[3];
+        a[4] = b1 * f[LW_H] + b2 * f[LW_CU] + b3 * s[4];
+#pragma unroll
+        for (int k = 0; k < 5; ++k) s[k] = F ? div * (base[k] + a[k]) : base[k] - div * a[k];
+        if (x + by != to) fetch(x + by);
+        if ((int)threadIdx.x < nl) {
+#pragma unroll
+          for (int k = 0; k < 5; ++k) at(x, LW_DQ + k, l) = s[k];
+        }
+      }
+    };
+    const int end = d == 2 ? 1 : 0;
+    walk(std::true_type{}, end, len, 1);
+    __syncwarp();
+    walk(std::false_type{}, len - 1 - end, -1, -1);
+  }
+  __syncthreads();
+  for (int t = threadIdx.x; t < len * nl; t += blockDim.x) {
+    const int l = d == 0 ? t / len : t % nl, x = d == 0 ? t % len : t / nl;
+    const long n = node(l, x);
+    const double ij = last ? B.s(F_INVJ, n) : 1.0;
+#pragma unroll
+    for (int k = 1; k <= 5; ++k) {
+      const double dq = at(x, LW_DQ + k - 1, l);
+      if (last)
+        B.v(F_Q, k, n) = B.v(F_Q, k, n) + dq / ij;
+      else
+        dqv(B, k, n) = dq;
+    }
+  }
+}
+// Dynamic shared memory of k_crank_lines for lines of `len` nodes.
+size_t crank_lines_smem(int len, int lpc) {
+  return (size_t)(len + 2) * (LW_NUM * lpc + 1 - (LW_NUM * lpc & 1)) * sizeof(double);
+}
+
+// The same through global memory, for lines that do not fit shared memory:
+// thread = one line of the updated box along
 // direction d (0: i, 1: j, 2: k).  The forward recurrence of the k lines
 // starts at ks1+1 and the backward one at ke1-1 (:352, :398), as in the
 // reference; along i and j they cover the whole line.

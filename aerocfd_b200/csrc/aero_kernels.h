@@ -61,6 +61,8 @@ __global__ void k_forces(const BlockView* __restrict__ blocks, const WallFace* _
 __global__ void k_residual_final_blocks(const BlockView* __restrict__ blocks, const double* __restrict__ part,
                                         int ctas, double* __restrict__ out7, unsigned* status);
 __global__ void k_crank_rhs(const BlockView* __restrict__ blocks);
+__global__ void k_crank_lines(const BlockView* __restrict__ blocks, int d, int lpc, double gamma, int last);
+size_t crank_lines_smem(int len, int lpc);
 __global__ void k_crank_sweep(const BlockView* __restrict__ blocks, int d, double gamma);
 __global__ void k_crank_update(const BlockView* __restrict__ blocks);
 __global__ void k_update_q0(const BlockView* __restrict__ blocks);

@@ -1259,13 +1259,34 @@ int do_getpri_all() {
 // crank2nd on nblk views (sub_timeadvancement_2ndcrank.f90): dual-time rhs,
 // dq = 0, the i, j, k line recurrences, q += dq/inv_j.
 int launch_crank(const BlockView* views, int nblk, long maxN, long maxN1, const Box* lines, const CaseConsts& cc) {
+  const long nl[3] = {(long)lines->ny() * lines->nz(), (long)lines->nx() * lines->nz(), (long)lines->nx() * lines->ny()};
+  const int len[3] = {lines->nx(), lines->ny(), lines->nz()};
+  const int dirs = cc.dimension == IFLAG_2D ? 2 : 3;  // 2-D (sub_timeadvancement_2ndcrank.f90:335): no k lines
+  // Lines in shared memory where four of them fit a CTA (lines of up to about
+  // 400 nodes): as many per CTA as spread the set over the SMs, at least the
+  // four that a 32-byte sector of the loads across the lines holds.
+  const size_t kSmem = 220 * 1024;
+  bool fit = true;
+  int lpc[3] = {4, 4, 4};
+  for (int d = 0; d < dirs; ++d) {
+    fit = fit && crank_lines_smem(len[d], 4) <= kSmem;
+    lpc[d] = (int)std::min<long>(32, std::max<long>(4, cdiv(nl[d] * nblk, kSms)));
+    while (lpc[d] > 4 && crank_lines_smem(len[d], lpc[d]) > kSmem) --lpc[d];
+  }
+  if (fit) {
+    CK(cudaFuncSetAttribute(k_crank_lines, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem));
+    for (int d = 0; d < dirs; ++d) {
+      PROF(P_CRANK, (k_crank_lines<<<dim3(cdiv(nl[d], lpc[d]), nblk), 256, crank_lines_smem(len[d], lpc[d]), g.stream>>>(
+                        views, d, lpc[d], cc.gamma, d == dirs - 1)));
+      CKL();
+    }
+    return AERO_OK;
+  }
   PROF(P_CRANK, (k_crank_rhs<<<dim3(cdiv(maxN1, 256), nblk), 256, 0, g.stream>>>(views)));
   CKL();
   PROF(P_CRANK, (k_fill<<<dim3(cdiv(maxN, 256), nblk), 256, 0, g.stream>>>(views, F_FVH, 5, 0.0)));
   CKL();
-  const long nl[3] = {(long)lines->ny() * lines->nz(), (long)lines->nx() * lines->nz(), (long)lines->nx() * lines->ny()};
-  // 2-D (sub_timeadvancement_2ndcrank.f90:335): no k lines
-  for (int d = 0; d < (cc.dimension == IFLAG_2D ? 2 : 3); ++d) {
+  for (int d = 0; d < dirs; ++d) {
     PROF(P_CRANK, (k_crank_sweep<<<dim3(cdiv(nl[d], 64), nblk), 64, 0, g.stream>>>(views, d, cc.gamma)));
     CKL();
   }
