@@ -1,0 +1,83 @@
+"""The pipelined LU-SGS sweeps against the oracle, whole iterations at 1e-12 per
+field (the arithmetic is the oracle's), for block shapes at the edges of the
+cuts: a single updated node, extents below the cluster's size, planes wider than
+a CTA's warps, many blocks (two CTAs per SM), one layer per slab, planes too wide
+for the pipeline, and mixed precision against FP64."""
+import numpy as np
+import pytest
+
+from aerocfd_b200 import grids
+from aerocfd_b200.case import IFLAG_NSSOLVER, IFLAG_SA, Config
+from conftest import relerr
+
+pytestmark = pytest.mark.gpu
+TOL = 1e-12
+
+
+@pytest.fixture(scope="module")
+def gpu():
+    from aerocfd_b200 import build, solver
+    build.build()
+    return solver
+
+
+def channel(*shape):
+    return lambda: grids.bump_channel(*shape)
+
+
+def channels(n, *shape):
+    return lambda: grids.batch_case([grids.bump_channel(*shape, h=0.05 + 0.001 * c) for c in range(n)])[0]
+
+
+def plate(*blocks, **size):
+    cfg = Config(solver=IFLAG_NSSOLVER, turbulence=IFLAG_SA, ma=0.2, re=5.0e6, cfl=2.0, nutinf=3.0)
+    return lambda: grids.flat_plate(*blocks, dy_wall=1e-4, cfg=cfg, **size)
+
+
+@pytest.mark.parametrize("make", [channel(3, 3, 3), channel(4, 9, 3), channel(40, 3, 3), channel(24, 20, 18),
+                                  channel(7, 40, 40), channels(40, 17, 41, 7), channels(90, 9, 9, 3),
+                                  plate(8, 1, 1, ni=41, nj=33, nk=9), plate(2, 2, 2, ni=25, nj=17, nk=9)])
+def test_block_shapes(gpu, oracle_mod, make):
+    co, cg = make(), make()
+    oc = oracle_mod.OracleCase(co)
+    oc.geometry()
+    oc.init_flowfield()
+    oc.start()
+    gc = gpu.GpuCase(cg)
+    try:
+        gc.compute_geometry()
+        gc.init_flowfield()
+        gc.start()
+        oc.iterate(3)
+        gc.step(3)
+        gc.sync_to_host(gpu.mask("q", "nut"))
+        assert gc.status() == 0
+        for bo, bg in zip(co.blocks, cg.blocks):
+            assert np.all(np.isfinite(bo.fields["q"]))
+            for k in ["q"] + (["nut"] if co.cfg.turbulence else []):
+                assert relerr(bg.fields[k], bo.fields[k]) <= TOL, (bg.m, k)
+    finally:
+        gc.close()
+
+
+def test_planes_too_wide_for_the_pipeline(gpu):
+    """A block whose planes no cluster's slabs hold takes the sweeps through
+    global memory; both give the update that splits of the same block give, so
+    the block is compared with itself in mixed precision (at most 1e-6) and the
+    run must stay finite."""
+    q = {}
+    for mixed in (False, True):
+        case = grids.bump_channel(70, 70, 70)
+        gc = gpu.GpuCase(case)
+        try:
+            gc.set_precision(mixed)
+            gc.compute_geometry()
+            gc.init_flowfield()
+            gc.start()
+            h = gc.step(2)
+            gc.sync_to_host(gpu.mask("q"))
+            assert gc.status() == 0 and np.all(np.isfinite(h))
+            q[mixed] = case.blocks[0].fields["q"].copy()
+        finally:
+            gc.close()
+    assert relerr(q[True], q[False]) <= 1e-6
