@@ -198,7 +198,11 @@ __global__ void k_aos_to_soa(const double* __restrict__ src, double* __restrict_
                              int nc, long plane);
 __global__ void k_soa_to_aos(const double* __restrict__ src, double* __restrict__ dst, long n,
                              int nc, long plane);
-__global__ void k_fill_plane(double* __restrict__ p, long n, double val);
+// freestream values of one block
+struct InitValues {
+  double q[5], pri[7], amu[3], dt, nut;
+};
+__global__ void k_init_flowfield(const BlockView* __restrict__ blocks, const InitValues* __restrict__ values, int sa);
 // one-time geometry
 __global__ void k_metric_pass1(const BlockView* __restrict__ blocks);
 __global__ void k_metric_pass2(const BlockView* __restrict__ blocks);

@@ -151,6 +151,9 @@ SlabFit slab_fit_for(const BlockView* hv, int nblk, int ncta, int rows);
 // sweep, the kernel's own bound.
 constexpr long kPollBudgetMax = 1L << 20;
 
+// Steps whose residuals aero_step keeps on their way to the host at a time.
+constexpr int kHistSteps = 256;
+
 struct State {
   bool inited = false;
   int device = 0;
@@ -237,7 +240,9 @@ struct State {
   bool retire = false;               // refresh the live flags from the status words every step
   double* d_out = nullptr;   // residual (7) + dt min/max (2)
   double* h_out = nullptr;   // pinned
+  double* h_hist = nullptr;  // pinned: residuals of kHistSteps steps (aero_step)
   unsigned* d_status = nullptr;
+  InitValues* d_init = nullptr;      // per-block freestream values (aero_init_flowfield)
   double* d_staging = nullptr;
   size_t staging_doubles = 0;
   double totalnodes = 0;
@@ -1529,6 +1534,7 @@ int aero_init(int device) {
   CK(cudaMemset(g.d_status, 0, 8 * sizeof(unsigned)));
   CK(cudaMalloc(&g.d_out, 16 * sizeof(double)));
   CK(cudaMallocHost(&g.h_out, 16 * sizeof(double)));
+  CK(cudaMallocHost(&g.h_hist, (size_t)kHistSteps * 7 * sizeof(double)));
   g.device = device;
   g.inited = true;
   return AERO_OK;
@@ -1567,6 +1573,7 @@ static void release_case() {
   cudaFree(g.d_resid_blocks); g.d_resid_blocks = nullptr;
   cudaFree(g.d_bstat); g.d_bstat = nullptr;
   cudaFree(g.d_live); g.d_live = nullptr;
+  cudaFree(g.d_init); g.d_init = nullptr;
   g.retire = false;
   g.nwall = 0;
   g.nquad = 0;
@@ -1585,6 +1592,7 @@ int aero_finalize(void) {
   cudaFree(g.d_status); g.d_status = nullptr;
   cudaFree(g.d_out); g.d_out = nullptr;
   cudaFreeHost(g.h_out); g.h_out = nullptr;
+  cudaFreeHost(g.h_hist); g.h_hist = nullptr;
   cudaStreamDestroy(g.stream); g.stream = nullptr;
   cudaStreamDestroy(g.stream2); g.stream2 = nullptr;
   cudaStreamDestroy(g.stream3); g.stream3 = nullptr;
@@ -2181,6 +2189,7 @@ int aero_finish_setup(void) {
     g.views[m].bstat = g.d_bstat + m;
     g.views[m].live = g.d_live + m;
   }
+  CK(cudaMalloc(&g.d_init, nb * sizeof(InitValues)));
   CK(cudaMalloc(&g.d_blocks, nb * sizeof(BlockView)));
   CK(cudaMalloc(&g.d_blocks_chain, nb * sizeof(BlockView)));
   if ((rc = upload_views())) return rc;
@@ -2754,34 +2763,20 @@ int aero_init_flowfield(void) {
   double t_0 = 1.0;
   bool sa = g.cc.turbulence == IFLAG_SA;
   double amu2 = sa ? 0.009 : 0.0;
-  double av[3] = {1.0, amu2, 1.0 + amu2};
+  std::vector<InitValues> val(nb);
   for (int m = 0; m < nb; ++m) {
     const CaseConsts& c = g.blocks[m].own_params ? g.blocks[m].cc : g.cc;
     const double dt0 = g.blocks[m].own_params ? g.blocks[m].params[5] : g.params[5];
-    double qv[5] = {c.d_0, c.d_0 * c.u_0 * std::cos(c.aoa), c.d_0 * c.u_0 * std::sin(c.aoa), 0.0,
-                    c.d_0 * t_0 * c.cv + 0.5 * c.d_0 * c.u_0 * c.u_0};
-    double pv[7] = {c.d_0, c.u_0 * std::cos(c.aoa), c.u_0 * std::sin(c.aoa), 0.0, c.p_0, t_0, c.c_0};
-    const BlockView& v = g.views[m];
-    long N = g.blocks[m].b.size();
-    auto put = [&](double* dst, double val) -> int {
-      PROF(P_FILL, (k_fill_plane<<<cdiv(N, 256), 256, 0, g.stream>>>(dst, N, val)));
-      CKL();
-      return AERO_OK;
-    };
-    for (int x = 0; x < 5; ++x) if ((rc = put(v.f[F_Q] + x * v.plane, qv[x]))) return rc;
-    for (int x = 0; x < 7; ++x) if ((rc = put(v.f[F_PRI] + x * v.plane, pv[x]))) return rc;
-    for (int x = 0; x < 3; ++x) if ((rc = put(v.f[F_AMU] + x * v.plane, av[x]))) return rc;
-    if ((rc = put(v.f[F_DT], dt0))) return rc;
-    for (int x = 0; x < 10; ++x)  // q0(l, c) = q(c) at both time levels (sub_init_flowfield.f90:78-82)
-      if ((rc = put(v.f[F_Q0] + x * v.plane, qv[x / 2]))) return rc;
-    if (sa) {
-      if ((rc = put(v.f[F_NUT], c.nutinf))) return rc;
-      if ((rc = put(v.f[F_SARHS], 0.0))) return rc;
-    }
-    for (int fid : {F_DUDX, F_VOR, F_TAO, F_RHSV, F_RHSI, F_RHS})
-      for (int x = 0; x < field_nc(fid); ++x)
-        if ((rc = put(v.f[fid] + x * v.plane, 0.0))) return rc;
+    val[m] = InitValues{{c.d_0, c.d_0 * c.u_0 * std::cos(c.aoa), c.d_0 * c.u_0 * std::sin(c.aoa), 0.0,
+                         c.d_0 * t_0 * c.cv + 0.5 * c.d_0 * c.u_0 * c.u_0},
+                        {c.d_0, c.u_0 * std::cos(c.aoa), c.u_0 * std::sin(c.aoa), 0.0, c.p_0, t_0, c.c_0},
+                        {1.0, amu2, 1.0 + amu2},
+                        dt0,
+                        c.nutinf};
   }
+  CK(cudaMemcpyAsync(g.d_init, val.data(), nb * sizeof(InitValues), cudaMemcpyHostToDevice, g.stream));
+  PROF(P_FILL, (k_init_flowfield<<<dim3(cdiv(g.max_box, 256), nb), 256, 0, g.stream>>>(g.d_blocks, g.d_init, sa)));
+  CKL();
   g.rhsi_ghosts_zero = true;
   CK(cudaStreamSynchronize(g.stream));
   return AERO_OK;
@@ -3012,19 +3007,25 @@ int aero_launch_count(unsigned long long* count) {
 int aero_step(int nsteps, double* resid_hist, double* dt_minmax) {
   int rc = need_setup();
   if (rc) return rc;
-  for (int s = 0; s < nsteps; ++s) {
-    bool last = (s == nsteps - 1);
-    if (last && dt_minmax != nullptr) {
-      if ((rc = do_iteration(true))) return rc;
-      if ((rc = do_getpri_all())) return rc;  // end of the time step (main.f90:434-447)
-      if ((rc = do_residual(g.d_out))) return rc;
-    } else if ((rc = run_step())) {
-      return rc;
+  // The residuals of up to kHistSteps steps cross the bus into pinned memory
+  // behind their steps; the host waits once per that many steps, so that it
+  // launches the next step while the device runs this one.
+  for (int s0 = 0; s0 < nsteps; s0 += kHistSteps) {
+    const int n = std::min(kHistSteps, nsteps - s0);
+    for (int s = s0; s < s0 + n; ++s) {
+      if (s == nsteps - 1 && dt_minmax != nullptr) {
+        if ((rc = do_iteration(true))) return rc;
+        if ((rc = do_getpri_all())) return rc;  // end of the time step (main.f90:434-447)
+        if ((rc = do_residual(g.d_out))) return rc;
+      } else if ((rc = run_step())) {
+        return rc;
+      }
+      if (resid_hist)
+        CK(cudaMemcpyAsync(g.h_hist + 7 * (s - s0), g.d_out, 7 * sizeof(double), cudaMemcpyDeviceToHost, g.stream));
     }
     if (resid_hist) {
-      CK(cudaMemcpyAsync(g.h_out, g.d_out, 7 * sizeof(double), cudaMemcpyDeviceToHost, g.stream));
       CK(cudaStreamSynchronize(g.stream));
-      std::memcpy(resid_hist + 7 * s, g.h_out, 7 * sizeof(double));
+      std::memcpy(resid_hist + 7 * s0, g.h_hist, (size_t)n * 7 * sizeof(double));
     }
   }
   if (dt_minmax) {
