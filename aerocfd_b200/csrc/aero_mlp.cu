@@ -46,62 +46,141 @@ __device__ __forceinline__ uint16_t to_bf16(float f) {  // round to nearest even
 }
 __device__ __forceinline__ float sigmoid(float z) { return 1.0f / (1.0f + expf(-z)); }
 
-// rows x cols FP32 (row stride ld_in) -> BF16 rows x ld_out, zero-padded
-// to ld_out columns and `rows_pad` rows.
-__global__ void k_pack_bf16(const float* __restrict__ in, int rows, int cols, int ld_in, uint16_t* __restrict__ out,
-                            int rows_pad, int ld_out) {
-  long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= (long)rows_pad * ld_out) return;
-  int r = (int)(i / ld_out), c = (int)(i % ld_out);
-  out[i] = (r < rows && c < cols) ? to_bf16(in[(long)r * ld_in + c]) : (uint16_t)0;
-}
-
-// z += b per column; h = bf16(silu(z)).
-__global__ void k_bias_silu(float* __restrict__ z, const float* __restrict__ b, uint16_t* __restrict__ h, int rows,
-                            int cols) {
-  long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
+// One batch of the network's inputs: rows idx[0 .. n) of src (idx null: rows 0 ..
+// n) in BF16 into h (rows x ld) and its transpose ht (ld x rows); rows past n are
+// zero, and the padding columns are zero from the start and never written.
+__global__ void k_load_inputs(const float* __restrict__ src, const int* __restrict__ idx, int n, int cols, int rows,
+                              int ld, uint16_t* __restrict__ h, uint16_t* __restrict__ ht) {
+  const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= (long)rows * cols) return;
-  float v = z[i] + b[i % cols];
-  z[i] = v;
-  h[i] = to_bf16(v * sigmoid(v));
+  const int r = (int)(i / cols), c = (int)(i % cols);
+  const uint16_t v = r < n ? to_bf16(src[(long)(idx ? idx[r] : r) * cols + c]) : (uint16_t)0;
+  h[(long)r * ld + c] = v;
+  ht[(long)c * rows + r] = v;
 }
 
-// Output layer: y = c + b; masked difference to the target; dy for the
-// backward GEMMs (BF16) and for the bias gradient (FP32); per-CTA loss sums.
-__global__ void k_out_loss(const float* __restrict__ c, const float* __restrict__ b, const float* __restrict__ t,
-                           int n_real, int n_out, int rows, int cols, float inv_count, float* __restrict__ y,
-                           uint16_t* __restrict__ dy, float* __restrict__ dyf, float* __restrict__ loss_part) {
-  long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  float l = 0.f;
-  if (i < (long)rows * cols) {
-    int r = (int)(i / cols), j = (int)(i % cols);
-    float v = c[i] + b[j];
-    y[i] = v;
-    float d = (r < n_real && j < n_out && t) ? v - t[(long)r * n_out + j] : 0.f;
-    l = d * d;
-    float g = 2.f * d * inv_count;
-    dy[i] = to_bf16(g);
-    dyf[i] = g;
+// y = c + b, the real rows and columns only.
+__global__ void k_outputs(const float* __restrict__ c, const float* __restrict__ b, int n, int n_out, int ld,
+                          float* __restrict__ y) {
+  const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= (long)n * n_out) return;
+  const int r = (int)(i / n_out), j = (int)(i % n_out);
+  y[i] = c[(long)r * ld + j] + b[j];
+}
+
+// Rows and columns of an elementwise CTA's tile, and its threads: 32 columns by
+// kTileRows rows, 32 x 32 threads, so that 32 warps hide the loads' and the
+// exponentials' latency.
+constexpr int kTileRows = 512;
+constexpr dim3 kTileThreads(32, 32);
+constexpr size_t kTileSmem = (size_t)kTileRows * 33 * sizeof(float);
+// Stores a tile's 32 columns (f[row][33]) in BF16 as rows of out (cols x rows).
+__device__ __forceinline__ void store_transposed(const float* f, int rows, uint16_t* __restrict__ out) {
+  const int lane = threadIdx.x;
+  for (int c = threadIdx.y; c < 32; c += 32)
+    for (int r = 2 * lane; r < kTileRows; r += 64) {
+      const uint32_t pair = (uint32_t)to_bf16(f[r * 33 + c]) | (uint32_t)to_bf16(f[(r + 1) * 33 + c]) << 16;
+      *(uint32_t*)(out + (long)(blockIdx.x * 32 + c) * rows + (long)blockIdx.y * kTileRows + r) = pair;
+    }
+}
+
+// Hidden layer, forward: z += b per column, h = bf16(silu(z)) and, for the weight
+// gradients (ht not null), its transpose.
+__global__ void __launch_bounds__(1024) k_activate(float* __restrict__ z, const float* __restrict__ b, int rows,
+                                                   int cols, uint16_t* __restrict__ h, uint16_t* __restrict__ ht) {
+  extern __shared__ float f[];
+  const int tx = threadIdx.x, col = blockIdx.x * 32 + tx;
+  const float bias = b[col];
+#pragma unroll 4
+  for (int r = threadIdx.y; r < kTileRows; r += 32) {
+    const long i = (long)(blockIdx.y * kTileRows + r) * cols + col;
+    const float v = z[i] + bias;
+    z[i] = v;
+    const float a = v * sigmoid(v);
+    h[i] = to_bf16(a);
+    f[r * 33 + tx] = a;
   }
-  __shared__ float sm[256];
-  sm[threadIdx.x] = l;
+  if (!ht) return;
   __syncthreads();
-  for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-    if (threadIdx.x < o) sm[threadIdx.x] += sm[threadIdx.x + o];
+  store_transposed(f, rows, ht);
+}
+
+// The elementwise parts of the backward pass: a CTA takes 32 columns of kTileRows
+// rows and forms the gradient g(row, column) there, its BF16 value row-major (the
+// GEMM for the layer below) and transposed (the weight gradient's GEMM), and its
+// column sums for the bias, summed over every eighth row, then over the eight,
+// in that order; the tiles' sums are added in order by the update.  One pass
+// over the inputs in place of four (silu', transpose, column sums and the FP32
+// copy they read: 52 us a layer of 8192 x 256).
+template <class G>
+__device__ __forceinline__ void column_pass(int rows, int cols, uint16_t* __restrict__ d, uint16_t* __restrict__ dt,
+                                            float* __restrict__ part, G g) {
+  extern __shared__ float f[];
+  __shared__ float sm[8][33];
+  const int tx = threadIdx.x, ty = threadIdx.y, col = blockIdx.x * 32 + tx, r0 = blockIdx.y * kTileRows;
+#pragma unroll 4
+  for (int r = ty; r < kTileRows; r += 32) {
+    const float v = g(r0 + r, col);
+    d[(long)(r0 + r) * cols + col] = to_bf16(v);
+    f[r * 33 + tx] = v;
+  }
+  __syncthreads();
+  if (ty < 8) {
+    float s = 0.f;
+#pragma unroll 16
+    for (int r = ty; r < kTileRows; r += 8) s += f[r * 33 + tx];
+    sm[ty][tx] = s;
+  }
+  store_transposed(f, rows, dt);
+  __syncthreads();
+  if (ty == 0) {
+    float t = 0.f;
+    for (int y = 0; y < 8; ++y) t += sm[y][tx];
+    part[(long)blockIdx.y * cols + col] = t;
+  }
+}
+
+// Hidden layer: dz = dh * silu'(z).
+__global__ void __launch_bounds__(1024) k_back_hidden(const float* __restrict__ dh, const float* __restrict__ z,
+                                                     int rows, int cols, uint16_t* __restrict__ dz,
+                                                     uint16_t* __restrict__ dzt, float* __restrict__ part) {
+  column_pass(rows, cols, dz, dzt, part, [&](int r, int c) {
+    const float zz = z[(long)r * cols + c], s = sigmoid(zz);
+    return dh[(long)r * cols + c] * (s * (1.f + zz * (1.f - s)));
+  });
+}
+
+// Output layer: y = c + b, the masked difference to the target and its gradient;
+// per-CTA sums of the squared differences.
+__global__ void __launch_bounds__(1024) k_back_output(const float* __restrict__ c, const float* __restrict__ b,
+                                                     const float* __restrict__ t, const int* __restrict__ idx,
+                                                     int n_real, int n_out, int rows, int cols, float inv_count,
+                                                     uint16_t* __restrict__ dy, uint16_t* __restrict__ dyt,
+                                                     float* __restrict__ part, float* __restrict__ loss_part) {
+  float l = 0.f;
+  column_pass(rows, cols, dy, dyt, part, [&](int r, int j) {
+    const float v = c[(long)r * cols + j] + b[j];
+    const float d = (r < n_real && j < n_out) ? v - t[(long)(idx ? idx[r] : r) * n_out + j] : 0.f;
+    l += d * d;
+    return 2.f * d * inv_count;
+  });
+  __shared__ float sm[1024];
+  const int tid = threadIdx.y * 32 + threadIdx.x;
+  sm[tid] = l;
+  __syncthreads();
+  for (int o = 512; o > 0; o >>= 1) {
+    if (tid < o) sm[tid] += sm[tid + o];
     __syncthreads();
   }
-  if (threadIdx.x == 0 && loss_part) loss_part[blockIdx.x] = sm[0];
+  if (tid == 0) loss_part[blockIdx.y * gridDim.x + blockIdx.x] = sm[0];
 }
 
-// dz = dh * silu'(z), BF16 for the GEMMs and FP32 for the bias gradient.
-__global__ void k_silu_back(const float* __restrict__ dh, const float* __restrict__ z, uint16_t* __restrict__ dz,
-                            float* __restrict__ dzf, long n) {
-  long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  float s = sigmoid(z[i]);
-  float g = dh[i] * (s * (1.f + z[i] * (1.f - s)));
-  dz[i] = to_bf16(g);
-  dzf[i] = g;
+// Sum of the loss parts of a step (one warp).
+__global__ void k_loss_sum(const float* __restrict__ part, int n, float* __restrict__ out) {
+  double s = 0.0;
+  for (int i = threadIdx.x; i < n; i += 32) s += part[i];
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+  if (threadIdx.x == 0) *out = (float)s;
 }
 
 // out[c][r] = in[r][c] for a rows x cols BF16 matrix (32 x 32 tiles).
@@ -120,61 +199,61 @@ __global__ void k_transpose_bf16(const uint16_t* __restrict__ in, int rows, int 
   }
 }
 
-// Column sums of a rows x cols FP32 matrix in a fixed order: CTA (x, y) sums
-// rows [y*chunk, (y+1)*chunk) of columns 32x..32x+31 into part[y][col].
-__global__ void k_colsum_part(const float* __restrict__ in, int rows, int cols, int chunk, float* __restrict__ part) {
-  int col = blockIdx.x * 32 + threadIdx.x;
-  int r0 = blockIdx.y * chunk, r1 = min(rows, r0 + chunk);
-  __shared__ float sm[8][33];
-  float s = 0.f;
-  if (col < cols)
-    for (int r = r0 + threadIdx.y; r < r1; r += blockDim.y) s += in[(long)r * cols + col];
-  sm[threadIdx.y][threadIdx.x] = s;
-  __syncthreads();
-  if (threadIdx.y == 0 && col < cols) {
-    float t = 0.f;
-    for (int y = 0; y < (int)blockDim.y; ++y) t += sm[y][threadIdx.x];
-    part[(long)blockIdx.y * cols + col] = t;
+// One layer's parameters (weights, then biases).
+struct LayerParams {
+  float *w, *mw, *vw, *gw, *b, *mb, *vb, *gb;
+  uint16_t *wb, *wt;  // BF16 copy of the weights and its transpose
+  int nin, nout;
+};
+// The layer's gradients from the weight GEMM's split-K partial tiles and the bias
+// column sums, each added in a fixed order: stored (train = 0), or (train = 1)
+// used by Adam (Kingma & Ba 2015) on the FP32 master parameters, which also
+// renews the BF16 weights and their transpose; one launch a layer in place of
+// five.
+__global__ void k_update_layer(LayerParams p, const float* __restrict__ wpart, int splits,
+                               const float* __restrict__ bpart, int chunks, int train, float lr, float b1, float b2,
+                               float c1, float c2, float eps) {
+  const long i = (long)blockIdx.x * blockDim.x + threadIdx.x, nw = (long)p.nin * p.nout;
+  if (i >= nw + p.nout) return;
+  const bool weight = i < nw;
+  const long j = weight ? i : i - nw, n = weight ? nw : p.nout;
+  const float* part = weight ? wpart : bpart;
+  float g = 0.f;
+#pragma unroll 8
+  for (int x = 0; x < (weight ? splits : chunks); ++x) g += part[(long)x * n + j];
+  if (!train) {
+    (weight ? p.gw : p.gb)[j] = g;
+    return;
   }
-}
-
-// Adam (Kingma & Ba 2015) on FP32 master parameters, with the BF16 copy.
-__global__ void k_adam(float* __restrict__ w, const float* __restrict__ g, float* __restrict__ m, float* __restrict__ v,
-                       uint16_t* __restrict__ wb, long n, float lr, float b1, float b2, float c1, float c2, float eps) {
-  long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  float gi = g[i];
-  float mi = b1 * m[i] + (1.f - b1) * gi;
-  float vi = b2 * v[i] + (1.f - b2) * gi * gi;
-  m[i] = mi;
-  v[i] = vi;
-  float wi = w[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
-  w[i] = wi;
-  if (wb) wb[i] = to_bf16(wi);
-}
-
-// Row gather of the training set into a batch (FP32), padded rows zero.
-__global__ void k_gather_rows(const float* __restrict__ src, const int* __restrict__ idx, int n_idx, int cols,
-                              float* __restrict__ dst, int rows_pad) {
-  long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= (long)rows_pad * cols) return;
-  int r = (int)(i / cols), c = (int)(i % cols);
-  dst[i] = r < n_idx ? src[(long)idx[r] * cols + c] : 0.f;
+  float *w = weight ? p.w : p.b, *m = weight ? p.mw : p.mb, *v = weight ? p.vw : p.vb;
+  const float mi = b1 * m[j] + (1.f - b1) * g;
+  const float vi = b2 * v[j] + (1.f - b2) * g * g;
+  m[j] = mi;
+  v[j] = vi;
+  const float wi = w[j] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+  w[j] = wi;
+  if (weight) {
+    const uint16_t b = to_bf16(wi);
+    p.wb[j] = b;
+    p.wt[(j % p.nin) * p.nout + j / p.nin] = b;
+  }
 }
 
 }  // namespace
 
-// C = A * B^T on the device; splits > 1 reduces the partial tiles into C with
-// `scratch` (splits * M * N floats).
-int gemm(const uint16_t* A, const uint16_t* B, float* C, int M, int N, int K, int splits, float* scratch,
-         unsigned* status, cudaStream_t st) {
+// The product C = A * B^T in `splits` partial tiles (changed to the number made),
+// one after another in C.
+int gemm_problem(GemmProblem& p, const uint16_t* A, const uint16_t* B, float* C, int M, int N, int K, int& splits) {
   if (M % kBM || N % kBN || K % kBK || splits < 1)
     return set_last_error(AERO_ERR_ARG, "tensor-core GEMM needs M, N multiples of 128 and K a multiple of 64");
-  int ktiles = K / kBK;
+  const int ktiles = K / kBK;
   if (splits > ktiles) splits = ktiles;
-  int klen = ((ktiles + splits - 1) / splits) * kBK;
+  const int klen = ((ktiles + splits - 1) / splits) * kBK;
   splits = (K + klen - 1) / klen;
-  dim3 grid(N / kBN, M / kBM, splits);
+  p = GemmProblem{A, B, C, M, N, K, klen, N / kBN * (M / kBM) * splits};
+  return AERO_OK;
+}
+int launch_gemms(const GemmProblem& p0, const GemmProblem& p1, unsigned* status, cudaStream_t st) {
   static int smem_dev = -1;  // device whose limit was raised (one device per process)
   int dev = 0;
   MCK(cudaGetDevice(&dev));
@@ -182,8 +261,22 @@ int gemm(const uint16_t* A, const uint16_t* B, float* C, int M, int N, int K, in
     MCK(cudaFuncSetAttribute(k_gemm_bf16, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGemmSmem));
     smem_dev = dev;
   }
-  k_gemm_bf16<<<grid, kGemmThreads, kGemmSmem, st>>>(A, B, splits > 1 ? scratch : C, M, N, K, klen, status);
+  k_gemm_bf16<<<p0.tiles + p1.tiles, kGemmThreads, kGemmSmem, st>>>(p0, p1, status);
   MCK(cudaGetLastError());
+  return AERO_OK;
+}
+int gemm_parts(const uint16_t* A, const uint16_t* B, float* C, int M, int N, int K, int& splits, unsigned* status,
+               cudaStream_t st) {
+  GemmProblem p;
+  int rc = gemm_problem(p, A, B, C, M, N, K, splits);
+  return rc ? rc : launch_gemms(p, GemmProblem{}, status, st);
+}
+// The same into C; splits > 1 adds the partial tiles from `scratch` (splits * M *
+// N floats).
+int gemm(const uint16_t* A, const uint16_t* B, float* C, int M, int N, int K, int splits, float* scratch,
+         unsigned* status, cudaStream_t st) {
+  int rc = gemm_parts(A, B, splits > 1 ? scratch : C, M, N, K, splits, status, st);
+  if (rc) return rc;
   if (splits > 1) {
     long n = (long)M * N;
     k_splitk_reduce<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(scratch, splits, n, C);
@@ -292,27 +385,43 @@ struct Net {
   int kin = 128, nout = 128;  // padded input and output widths
   std::vector<Layer> L;       // depth hidden layers, then the output layer
   std::vector<uint16_t*> h;   // h[0] input, h[l] = silu(z[l-1]); BF16 batch x width
+  std::vector<uint16_t*> ht;  // their transposes
   std::vector<float*> z;      // pre-activations, FP32
-  float *c_out = nullptr, *y = nullptr, *dyf = nullptr, *dh = nullptr, *dzf = nullptr;
-  uint16_t *dy = nullptr, *dz = nullptr, *tA = nullptr, *tB = nullptr;
-  float *scratch = nullptr, *cpart = nullptr, *lpart = nullptr, *lhist = nullptr;
+  float *c_out = nullptr, *y = nullptr, *dh = nullptr;
+  uint16_t *d = nullptr, *dt = nullptr;  // a layer's gradient and its transpose
+  float *scratch = nullptr, *cpart = nullptr, *lpart = nullptr;
   float *xb = nullptr, *tb = nullptr, *xall = nullptr, *tall = nullptr;
-  int* idx = nullptr;
+  int* perm[2] = {nullptr, nullptr};  // row order of an epoch and of the next
   unsigned* status = nullptr;
   long n_all = 0;
   int adam_t = 0;
   std::vector<void*> allocs;
+  char* arena = nullptr;  // rest of the newest allocation
+  size_t arena_left = 0;
 } g_net;
 
 constexpr int kSplitMax = 32;
-constexpr int kColChunk = 512;
 
+// The network's arrays share a few device allocations (each of at least
+// kArenaBytes); an array starts on a 256-byte boundary.
+constexpr size_t kArenaBytes = (size_t)256 << 20;
 template <class T>
 int alloc(T*& p, size_t n) {
   p = nullptr;
-  if (cudaMalloc(&p, n * sizeof(T)) != cudaSuccess) return set_last_error(AERO_ERR_NOMEM, "warm-start network: device allocation failed");
-  g_net.allocs.push_back(p);
-  cudaMemset(p, 0, n * sizeof(T));
+  const size_t bytes = (n * sizeof(T) + 255) / 256 * 256;
+  if (bytes > g_net.arena_left) {
+    void* a = nullptr;
+    const size_t size = std::max(bytes, kArenaBytes);
+    if (cudaMalloc(&a, size) != cudaSuccess)
+      return set_last_error(AERO_ERR_NOMEM, "warm-start network: device allocation failed");
+    g_net.allocs.push_back(a);
+    cudaMemset(a, 0, size);
+    g_net.arena = (char*)a;
+    g_net.arena_left = size;
+  }
+  p = (T*)g_net.arena;
+  g_net.arena += bytes;
+  g_net.arena_left -= bytes;
   return AERO_OK;
 }
 
@@ -320,6 +429,8 @@ void release() {
   for (void* p : g_net.allocs) cudaFree(p);
   cudaFree(g_net.xall);
   cudaFree(g_net.tall);
+  cudaFree(g_net.perm[0]);
+  cudaFree(g_net.perm[1]);
   g_net = Net{};
 }
 
@@ -327,14 +438,6 @@ unsigned cdiv(long a, long b) { return (unsigned)((a + b - 1) / b); }
 
 int transpose(const uint16_t* in, int rows, int cols, uint16_t* out) {
   k_transpose_bf16<<<dim3(cols / 32, rows / 32), dim3(32, 8)>>>(in, rows, cols, out);
-  MCK(cudaGetLastError());
-  return AERO_OK;
-}
-int colsum(const float* in, int rows, int cols, float* out) {
-  int chunks = (rows + kColChunk - 1) / kColChunk;
-  k_colsum_part<<<dim3(cdiv(cols, 32), chunks), dim3(32, 8)>>>(in, rows, cols, kColChunk, g_net.cpart);
-  MCK(cudaGetLastError());
-  k_splitk_reduce<<<cdiv(cols, 256), 256>>>(g_net.cpart, chunks, cols, out);
   MCK(cudaGetLastError());
   return AERO_OK;
 }
@@ -346,66 +449,61 @@ int refresh_transposes() {
   return AERO_OK;
 }
 
-// Forward pass of the current batch (xb: batch x n_in FP32); with targets tb,
-// the loss parts and dy for the backward pass.
-int forward(int n_real, bool with_loss) {
+// Forward pass of the rows idx[0 .. n) (null: 0 .. n) of x, to c_out (without the
+// output layer's bias); with_back also leaves what backward reads.
+int forward(const float* x, const int* idx, int n, bool with_back) {
   Net& N = g_net;
   const int B = N.batch;
-  int rc;
-  k_pack_bf16<<<cdiv((long)B * N.kin, 256), 256>>>(N.xb, n_real, N.n_in, N.n_in, N.h[0], B, N.kin);
+  int rc, one = 1;
+  k_load_inputs<<<cdiv((long)B * N.n_in, 256), 256>>>(x, idx, n, N.n_in, B, N.kin, N.h[0], N.ht[0]);
   MCK(cudaGetLastError());
   for (int l = 0; l < N.depth; ++l) {
-    if ((rc = gemm(N.h[l], N.L[l].wb, N.z[l], B, N.width, N.L[l].nin, 1, N.scratch, N.status, 0))) return rc;
-    k_bias_silu<<<cdiv((long)B * N.width, 256), 256>>>(N.z[l], N.L[l].b, N.h[l + 1], B, N.width);
+    if ((rc = gemm_parts(N.h[l], N.L[l].wb, N.z[l], B, N.width, N.L[l].nin, one, N.status, 0))) return rc;
+    k_activate<<<dim3(N.width / 32, B / kTileRows), kTileThreads, kTileSmem>>>(N.z[l], N.L[l].b, B, N.width, N.h[l + 1],
+                                                                               with_back ? N.ht[l + 1] : nullptr);
     MCK(cudaGetLastError());
   }
-  Layer& O = N.L[N.depth];
-  if ((rc = gemm(N.h[N.depth], O.wb, N.c_out, B, N.nout, N.width, 1, N.scratch, N.status, 0))) return rc;
-  float inv = 1.0f / ((float)n_real * (float)N.n_out);
-  k_out_loss<<<cdiv((long)B * N.nout, 256), 256>>>(N.c_out, O.b, with_loss ? N.tb : nullptr, n_real, N.n_out, B,
-                                                    N.nout, inv, N.y, N.dy, N.dyf, N.lpart);
-  MCK(cudaGetLastError());
-  return AERO_OK;
+  return gemm_parts(N.h[N.depth], N.L[N.depth].wb, N.c_out, B, N.nout, N.width, one, N.status, 0);
 }
 
-// Gradients of the loss of the last forward pass into every layer's gw, gb.
-int backward() {
-  Net& N = g_net;
-  const int B = N.batch;
-  int rc;
-  int split = std::min(kSplitMax, B / 512);
-  Layer& O = N.L[N.depth];
-  if ((rc = transpose(N.dy, B, N.nout, N.tA))) return rc;
-  if ((rc = transpose(N.h[N.depth], B, N.width, N.tB))) return rc;
-  if ((rc = gemm(N.tA, N.tB, O.gw, N.nout, N.width, B, split, N.scratch, N.status, 0))) return rc;
-  if ((rc = colsum(N.dyf, B, N.nout, O.gb))) return rc;
-  if ((rc = gemm(N.dy, O.wt, N.dh, B, N.width, N.nout, 1, N.scratch, N.status, 0))) return rc;
-  for (int l = N.depth - 1; l >= 0; --l) {
-    Layer& Ly = N.L[l];
-    k_silu_back<<<cdiv((long)B * N.width, 256), 256>>>(N.dh, N.z[l], N.dz, N.dzf, (long)B * N.width);
-    MCK(cudaGetLastError());
-    if ((rc = transpose(N.dz, B, N.width, N.tA))) return rc;
-    if ((rc = transpose(N.h[l], B, Ly.nin, N.tB))) return rc;
-    if ((rc = gemm(N.tA, N.tB, Ly.gw, N.width, Ly.nin, B, split, N.scratch, N.status, 0))) return rc;
-    if ((rc = colsum(N.dzf, B, N.width, Ly.gb))) return rc;
-    if (l > 0 && (rc = gemm(N.dz, Ly.wt, N.dh, B, Ly.nin, N.width, 1, N.scratch, N.status, 0))) return rc;
-  }
-  return AERO_OK;
-}
+int loss_parts() { return g_net.nout / 32 * (g_net.batch / kTileRows); }
 
-int adam_step(float lr) {
+// Backward pass of the last forward with the targets t (rows as forward's): the
+// loss parts and, layer by layer, the gradients into gw, gb or (train) an Adam
+// step with them.
+int backward(const float* t, const int* idx, int n, bool train, float lr) {
   Net& N = g_net;
-  ++N.adam_t;
+  const int B = N.batch, chunks = B / kTileRows;
+  int rc, one = 1;
   const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
-  float c1 = 1.f - std::pow(b1, (float)N.adam_t), c2 = 1.f - std::pow(b2, (float)N.adam_t);
-  for (Layer& l : N.L) {
-    long nw = (long)l.nin * l.nout;
-    k_adam<<<cdiv(nw, 256), 256>>>(l.w, l.gw, l.mw, l.vw, l.wb, nw, lr, b1, b2, c1, c2, eps);
+  float c1 = 1.f, c2 = 1.f;
+  if (train) {
+    ++N.adam_t;
+    c1 = 1.f - std::pow(b1, (float)N.adam_t);
+    c2 = 1.f - std::pow(b2, (float)N.adam_t);
+  }
+  for (int l = N.depth; l >= 0; --l) {
+    Layer& y = N.L[l];
+    const dim3 grid(y.nout / 32, chunks);
+    if (l == N.depth)
+      k_back_output<<<grid, kTileThreads, kTileSmem>>>(N.c_out, y.b, t, idx, n, N.n_out, B, y.nout, 1.0f / ((float)n * (float)N.n_out),
+                                     N.d, N.dt, N.cpart, N.lpart);
+    else
+      k_back_hidden<<<grid, kTileThreads, kTileSmem>>>(N.dh, N.z[l], B, y.nout, N.d, N.dt, N.cpart);
     MCK(cudaGetLastError());
-    k_adam<<<cdiv(l.nout, 256), 256>>>(l.b, l.gb, l.mb, l.vb, nullptr, l.nout, lr, b1, b2, c1, c2, eps);
+    // the weight gradient and, by this layer's weights before their update, the
+    // gradient of the layer below
+    int splits = std::min(kSplitMax, B / 512);
+    GemmProblem gw, dh;
+    if ((rc = gemm_problem(gw, N.dt, N.ht[l], N.scratch, y.nout, y.nin, B, splits))) return rc;
+    if (l > 0 && (rc = gemm_problem(dh, N.d, y.wt, N.dh, B, y.nin, y.nout, one))) return rc;
+    if ((rc = launch_gemms(gw, dh, N.status, 0))) return rc;
+    const LayerParams p{y.w, y.mw, y.vw, y.gw, y.b, y.mb, y.vb, y.gb, y.wb, y.wt, y.nin, y.nout};
+    k_update_layer<<<cdiv((long)y.nin * y.nout + y.nout, 256), 256>>>(p, N.scratch, splits, N.cpart, chunks, train,
+                                                                     lr, b1, b2, c1, c2, eps);
     MCK(cudaGetLastError());
   }
-  return refresh_transposes();
+  return AERO_OK;
 }
 
 int check_status() {
@@ -473,22 +571,24 @@ int aero_mlp_create(int n_in, int n_out, int width, int depth, int batch, unsign
     N.L.push_back(y);
   }
   N.h.resize(depth + 1);
+  N.ht.resize(depth + 1);
   N.z.resize(depth);
-  if ((rc = alloc(N.h[0], (size_t)batch * N.kin))) return rc;
-  for (int l = 1; l <= depth; ++l)
-    if ((rc = alloc(N.h[l], (size_t)batch * width))) return rc;
+  for (int l = 0; l <= depth; ++l) {
+    const size_t n = (size_t)batch * (l == 0 ? N.kin : width);
+    if ((rc = alloc(N.h[l], n)) || (rc = alloc(N.ht[l], n))) return rc;
+  }
   for (int l = 0; l < depth; ++l)
     if ((rc = alloc(N.z[l], (size_t)batch * width))) return rc;
   size_t wmax = (size_t)std::max(width, 128);
-  if ((rc = alloc(N.c_out, (size_t)batch * N.nout)) || (rc = alloc(N.y, (size_t)batch * N.nout)) ||
-      (rc = alloc(N.dyf, (size_t)batch * N.nout)) || (rc = alloc(N.dy, (size_t)batch * N.nout)) ||
-      (rc = alloc(N.dh, (size_t)batch * width)) || (rc = alloc(N.dzf, (size_t)batch * width)) ||
-      (rc = alloc(N.dz, (size_t)batch * width)) || (rc = alloc(N.tA, (size_t)batch * wmax)) ||
-      (rc = alloc(N.tB, (size_t)batch * wmax)) || (rc = alloc(N.scratch, (size_t)kSplitMax * wmax * wmax)) ||
-      (rc = alloc(N.cpart, (size_t)(batch / kColChunk + 1) * wmax)) ||
-      (rc = alloc(N.lpart, (size_t)cdiv((long)batch * N.nout, 256))) || (rc = alloc(N.xb, (size_t)batch * n_in)) ||
-      (rc = alloc(N.tb, (size_t)batch * n_out)) || (rc = alloc(N.idx, (size_t)batch)) || (rc = alloc(N.status, 1)))
+  if ((rc = alloc(N.c_out, (size_t)batch * N.nout)) || (rc = alloc(N.y, (size_t)batch * n_out)) ||
+      (rc = alloc(N.dh, (size_t)batch * width)) || (rc = alloc(N.d, (size_t)batch * wmax)) ||
+      (rc = alloc(N.dt, (size_t)batch * wmax)) || (rc = alloc(N.scratch, (size_t)kSplitMax * wmax * wmax)) ||
+      (rc = alloc(N.cpart, (size_t)(batch / kTileRows) * wmax)) || (rc = alloc(N.lpart, (size_t)loss_parts())) ||
+      (rc = alloc(N.xb, (size_t)batch * n_in)) || (rc = alloc(N.tb, (size_t)batch * n_out)) ||
+      (rc = alloc(N.status, 1)))
     return rc;
+  for (auto k : {(const void*)k_activate, (const void*)k_back_hidden, (const void*)k_back_output})
+    MCK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTileSmem));
   if ((rc = refresh_transposes())) return rc;
   MCK(cudaDeviceSynchronize());
   N.ok = true;
@@ -527,12 +627,11 @@ int aero_mlp_gradients(const float* x, const float* t, int n, float* loss, float
   Net& N = g_net;
   if (!N.ok) return set_last_error(AERO_ERR_STATE, "aero_mlp_create has not been called");
   if (n < 1 || n > N.batch) return set_last_error(AERO_ERR_ARG, "aero_mlp_gradients: 1 <= n <= batch");
-  MCK(cudaMemset(N.xb, 0, (size_t)N.batch * N.n_in * 4));
   MCK(cudaMemcpy(N.xb, x, (size_t)n * N.n_in * 4, cudaMemcpyHostToDevice));
   MCK(cudaMemcpy(N.tb, t, (size_t)n * N.n_out * 4, cudaMemcpyHostToDevice));
   int rc;
-  if ((rc = forward(n, true)) || (rc = backward())) return rc;
-  int np = (int)cdiv((long)N.batch * N.nout, 256);
+  if ((rc = forward(N.xb, nullptr, n, true)) || (rc = backward(N.tb, nullptr, n, false, 0.f))) return rc;
+  int np = loss_parts();
   std::vector<float> lp(np);
   MCK(cudaMemcpy(lp.data(), N.lpart, np * 4, cudaMemcpyDeviceToHost));
   double sum = 0;
@@ -556,9 +655,13 @@ int aero_mlp_train(const float* x, const float* t, long long n, int steps, float
   if (n < N.batch || steps < 1) return set_last_error(AERO_ERR_ARG, "aero_mlp_train: n >= batch and steps >= 1");
   int rc = AERO_OK;
   if (N.n_all != n) {
-    if (N.xall) { cudaFree(N.xall); cudaFree(N.tall); N.xall = N.tall = nullptr; }
+    cudaFree(N.xall); cudaFree(N.tall); cudaFree(N.perm[0]); cudaFree(N.perm[1]);
+    N.xall = N.tall = nullptr;
+    N.perm[0] = N.perm[1] = nullptr;
+    N.n_all = 0;
     MCK(cudaMalloc(&N.xall, (size_t)n * N.n_in * 4));
     MCK(cudaMalloc(&N.tall, (size_t)n * N.n_out * 4));
+    for (int k = 0; k < 2; ++k) MCK(cudaMalloc(&N.perm[k], (size_t)n * sizeof(int)));
     N.n_all = n;
   }
   MCK(cudaMemcpy(N.xall, x, (size_t)n * N.n_in * 4, cudaMemcpyHostToDevice));
@@ -569,8 +672,10 @@ int aero_mlp_train(const float* x, const float* t, long long n, int steps, float
   std::vector<int> perm(n);
   for (long long i = 0; i < n; ++i) perm[i] = (int)i;
   long long pos = n;
-  std::vector<int> bidx(N.batch);
-  int np = (int)cdiv((long)N.batch * N.nout, 256);
+  // An epoch's row order crosses the bus once, in stream order, into the buffer
+  // of the epoch before last, whose steps are over by then; nothing in the loop
+  // waits for the device, so the host shuffles and launches ahead of it.
+  int epoch = -1;
   for (int step = 0; step < steps && !rc; ++step) {
     if (pos + N.batch > n) {  // new epoch: Fisher-Yates shuffle
       for (long long i = n - 1; i > 0; --i) {
@@ -578,17 +683,17 @@ int aero_mlp_train(const float* x, const float* t, long long n, int steps, float
         std::swap(perm[i], perm[j]);
       }
       pos = 0;
+      ++epoch;
+      if (cudaMemcpyAsync(N.perm[epoch & 1], perm.data(), (size_t)n * sizeof(int), cudaMemcpyHostToDevice, 0) !=
+          cudaSuccess) {
+        rc = set_last_error(AERO_ERR_CUDA, "aero_mlp_train: copy of the row order failed");
+        break;
+      }
     }
-    std::copy(perm.begin() + pos, perm.begin() + pos + N.batch, bidx.begin());
+    const int* idx = N.perm[epoch & 1] + pos;
     pos += N.batch;
-    if (cudaMemcpy(N.idx, bidx.data(), (size_t)N.batch * 4, cudaMemcpyHostToDevice) != cudaSuccess) {
-      rc = set_last_error(AERO_ERR_CUDA, "aero_mlp_train: copy of the batch indices failed");
-      break;
-    }
-    k_gather_rows<<<cdiv((long)N.batch * N.n_in, 256), 256>>>(N.xall, N.idx, N.batch, N.n_in, N.xb, N.batch);
-    k_gather_rows<<<cdiv((long)N.batch * N.n_out, 256), 256>>>(N.tall, N.idx, N.batch, N.n_out, N.tb, N.batch);
-    if ((rc = forward(N.batch, true)) || (rc = backward()) || (rc = adam_step(lr))) break;
-    k_splitk_reduce<<<1, 32>>>(N.lpart, np, 1, dhist + step);  // sum of squared errors of the step
+    if ((rc = forward(N.xall, idx, N.batch, true)) || (rc = backward(N.tall, idx, N.batch, true, lr))) break;
+    k_loss_sum<<<1, 32>>>(N.lpart, loss_parts(), dhist + step);  // sum of squared errors of the step
   }
   if (!rc && cudaDeviceSynchronize() != cudaSuccess) rc = set_last_error(AERO_ERR_CUDA, "aero_mlp_train failed");
   if (!rc && loss_hist) {
@@ -606,15 +711,13 @@ int aero_mlp_predict(const float* x, long long n, float* y) {
   Net& N = g_net;
   if (!N.ok) return set_last_error(AERO_ERR_STATE, "aero_mlp_create has not been called");
   int rc;
-  std::vector<float> yb((size_t)N.batch * N.nout);
   for (long long r0 = 0; r0 < n; r0 += N.batch) {
     int m = (int)std::min<long long>(N.batch, n - r0);
-    MCK(cudaMemset(N.xb, 0, (size_t)N.batch * N.n_in * 4));
     MCK(cudaMemcpy(N.xb, x + r0 * N.n_in, (size_t)m * N.n_in * 4, cudaMemcpyHostToDevice));
-    if ((rc = forward(m, false))) return rc;
-    MCK(cudaMemcpy(yb.data(), N.y, yb.size() * 4, cudaMemcpyDeviceToHost));
-    for (int r = 0; r < m; ++r)
-      for (int c = 0; c < N.n_out; ++c) y[(r0 + r) * N.n_out + c] = yb[(size_t)r * N.nout + c];
+    if ((rc = forward(N.xb, nullptr, m, false))) return rc;
+    k_outputs<<<cdiv((long)m * N.n_out, 256), 256>>>(N.c_out, N.L[N.depth].b, m, N.n_out, N.nout, N.y);
+    MCK(cudaGetLastError());
+    MCK(cudaMemcpy(y + r0 * N.n_out, N.y, (size_t)m * N.n_out * 4, cudaMemcpyDeviceToHost));
   }
   return check_status();
 }

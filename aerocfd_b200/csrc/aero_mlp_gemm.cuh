@@ -1,7 +1,7 @@
 // BF16 GEMM on the 5th-generation tensor cores (tcgen05, sm_100a) for the
 // warm-start network: C[M x N] (FP32) = A[M x K] * B[N x K]^T, A and B
 // row-major BF16 (K-major operands), M and N multiples of 128, K a multiple of
-// 64.  Split-K: blockIdx.z = s covers K rows [s*klen, (s+1)*klen) and writes
+// 64.  Split-K: part s covers K rows [s*klen, (s+1)*klen) and writes
 // its partial tile to C + s*M*N (a fixed-order reduction adds the partials).
 //
 // Per CTA (128 threads): one 128 x 128 FP32 accumulator in tensor memory (128
@@ -79,19 +79,34 @@ __device__ __forceinline__ bool gemm_wait(uint32_t bar, unsigned parity, long bu
 // issues the tile's MMAs and commits them on the stage's mbarrier; then the
 // stage of tile t-1 is refilled with tile t+S-1 once that tile's commit has
 // arrived (its MMAs have read the stage).
-__global__ void __launch_bounds__(kGemmThreads, 2) k_gemm_bf16(const uint16_t* __restrict__ A, const uint16_t* __restrict__ B,
-                                                  float* __restrict__ C, int M, int N, int K, int klen,
-                                                  unsigned* status) {
+//
+// A launch takes one product or two independent ones (a layer's weight gradient
+// and the gradient of the layer below: 64 and 128 tiles of 8192 x 256 layers,
+// which together fill the SMs' two CTAs each), the first p.tiles CTAs the first.
+struct GemmProblem {
+  const uint16_t *A = nullptr, *B = nullptr;
+  float* C = nullptr;
+  int M = 0, N = 0, K = 0, klen = 0, tiles = 0;
+};
+__global__ void __launch_bounds__(kGemmThreads, 2) k_gemm_bf16(GemmProblem p0, GemmProblem p1, unsigned* status) {
   constexpr int S = kGemmStages;
   extern __shared__ uint8_t gemm_smem[];
   __shared__ __align__(8) unsigned long long bar[S];
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_flag;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int m0 = blockIdx.y * kBM, n0 = blockIdx.x * kBN;
-  const int kbeg = blockIdx.z * klen, kend = min(K, kbeg + klen);
+  const bool first = (int)blockIdx.x < p0.tiles;
+  const uint16_t* __restrict__ A = first ? p0.A : p1.A;
+  const uint16_t* __restrict__ B = first ? p0.B : p1.B;
+  float* __restrict__ C = first ? p0.C : p1.C;
+  const int M = first ? p0.M : p1.M, N = first ? p0.N : p1.N, K = first ? p0.K : p1.K;
+  const int klen = first ? p0.klen : p1.klen;
+  // tile: column, then row, then K part
+  const int tile = (int)blockIdx.x - (first ? 0 : p0.tiles), nn = N / kBN, nm = M / kBM;
+  const int n0 = tile % nn * kBN, m0 = tile / nn % nm * kBM, part = tile / nn / nm;
+  const int kbeg = part * klen, kend = min(K, kbeg + klen);
   const int nt = (kend - kbeg) / kBK;  // K-tiles of this CTA (K and klen are multiples of kBK)
-  float* Cs = C + (long)blockIdx.z * M * N;
+  float* Cs = C + (long)part * M * N;
   // stage s: A tile at base + s * 32 KB, B tile 16 KB after it
   const uint32_t raw = smem_addr(gemm_smem);
   const uint32_t base_s = (raw + 1023u) & ~1023u;
