@@ -230,3 +230,47 @@ def test_division_by_a_reciprocal_in_two_words(tmp_path):
                     os.path.join(ROOT, "aerocfd_b200", "csrc"), str(src), "-o", str(exe)], check=True)
     out = subprocess.run([str(exe)], capture_output=True, text=True)
     assert out.returncode == 0, out.stdout
+
+
+@pytest.mark.skipif(shutil.which("g++") is None, reason="needs a C++ compiler")
+def test_division_by_a_rounded_reciprocal(tmp_path):
+    """div_rn_lean equals IEEE division to the bit (zeros: in value) inside its
+    operand range, at the range's bounds, outside it and for special values."""
+    head, _ = DIV.split("int main() {")
+    src = tmp_path / "lean.cpp"
+    src.write_text(head + r"""
+int main() {
+  std::mt19937_64 g(7);
+  std::uniform_real_distribution<double> u(1.0, 2.0);
+  long bad = 0;
+  auto num = [&](int e) { return std::ldexp(u(g), e) * ((g() & 1) ? -1 : 1); };
+  auto one = [&](double a, double b) {
+    const double q = aero::div_rn_lean(a, b, 1.0 / b), t = a / b;
+    if (std::memcmp(&q, &t, 8) && !(std::isnan(q) && std::isnan(t)) && !(q == 0 && t == 0)) ++bad;
+  };
+  for (int ea = -1060; ea <= 1020; ea += 13)
+    for (int eb = -1060; eb <= 1020; eb += 17)
+      for (int x = 0; x < 20; ++x) one(num(ea), num(eb));
+  const int edge[] = {-481, -480, -479, 479, 480, 481};
+  for (int ea : edge)
+    for (int eb : edge) {
+      for (int x = 0; x < 50; ++x) one(num(ea), num(eb));
+      one(std::ldexp(1.0, ea), std::ldexp(-1.0, eb));
+    }
+  for (long x = 0; x < 2000000; ++x) {  // quotients next to a rounding midpoint
+    const double q = u(g), b = num((int)(g() % 60) - 30);
+    double a = (double)((long double)(q + std::ldexp(1.0, -53)) * (long double)b);
+    for (int k = (int)(g() % 3); k > 0; --k) a = std::nextafter(a, (g() & 1) ? INFINITY : -INFINITY);
+    one(a, b);
+  }
+  for (double b : {3.0, -3.0, 0.0, -0.0, 1e-300, 1e300, (double)INFINITY, (double)NAN})
+    for (double a : {0.0, -0.0, 1.0, 1e-310, 1e308, (double)INFINITY, (double)-INFINITY, (double)NAN}) one(a, b);
+  std::printf("bad=%ld\n", bad);
+  return bad != 0;
+}
+""")
+    exe = tmp_path / "lean"
+    subprocess.run(["g++", "-O2", "-std=c++17", "-ffp-contract=off", "-I",
+                    os.path.join(ROOT, "aerocfd_b200", "csrc"), str(src), "-o", str(exe)], check=True)
+    out = subprocess.run([str(exe)], capture_output=True, text=True)
+    assert out.returncode == 0, out.stdout
