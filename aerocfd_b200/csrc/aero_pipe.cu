@@ -170,21 +170,50 @@ __global__ void k_pipe_index(const BlockView* __restrict__ blocks) {
   P.sa_rec[(long)kPipeSaRec * pos + SW_NBR] = word;
 }
 
+#ifdef __CUDACC__  // (the order's tables above also build as host code, for their test)
+// A warp's 32 records from shared memory to their places, CHUNKS 16-byte chunks
+// from word `word` on, chunk c of lane r's record at sm[r * CHUNKS + c]; p is the
+// lane's position, or -1.  Consecutive lanes store consecutive chunks, so a store
+// covers whole runs of records instead of 16 bytes in each of 32 (which the L2
+// counted as 17.4 million sectors on the plate, 2.5 times the bytes).  A chunk
+// `half` keeps its upper word.
+template <int CHUNKS>
+__device__ __forceinline__ void store_records(const double2* sm, double* base, int words, int word, int p, int half) {
+  __syncwarp();
+  const int lane = (int)(threadIdx.x & 31);
+#pragma unroll
+  for (int x = lane; x < 32 * CHUNKS; x += 32) {
+    const int r = x / CHUNKS, c = x - r * CHUNKS;
+    const int pr = __shfl_sync(0xffffffffu, p, r);
+    if (pr < 0) continue;
+    double* to = base + (long)words * pr + word + 2 * c;
+    if (c == half)
+      to[0] = sm[x].x;
+    else
+      *reinterpret_cast<double2*>(to) = sm[x];
+  }
+}
+
 // Per updated node what its blocks are made of: the
 // spectral radii (sub_timeadvancement_1stimplicit.f90:108-156) and calc_jm's
 // common terms (sub_timeadvancement_jac.f90:17-62).  It reads q, the primitives
 // and the metrics only, so it runs beside the flux and time-step kernels.  The
 // nodes are taken in box order: the loads run along the rows of the box, and a
-// record is written by one thread whatever its place.
+// warp writes its records one after another (store_records), wherever they lie.
+// Plate (0.72 million nodes): 95 us for 320 MB, 138 with each thread storing its
+// own record.
 __global__ void k_pipe_recs(const BlockView* __restrict__ blocks, CaseConsts cc_launch) {
   const BlockView& B = blocks[blockIdx.y];
   if (B.retired()) return;
   const CaseConsts& cc = B.ccb ? *B.ccb : cc_launch;
   const int u = (int)(blockIdx.x * blockDim.x + threadIdx.x);
-  if (u >= B.b1.size()) return;
-  const long n = box_node(B, u);
-  const int p = B.pipe.at[u];
-  double2* rec = reinterpret_cast<double2*>(B.pipe.rec + (long)kPipeRec * p);
+  if (u - (int)threadIdx.x >= B.b1.size()) return;  // the whole CTA
+  constexpr int CH = PW_NBR / 2;
+  __shared__ double2 sm[128 * CH];
+  const bool act = u < B.b1.size();
+  const long n = box_node(B, act ? u : 0);
+  const int p = act ? B.pipe.at[u] : -1;
+  double2* rec = sm + threadIdx.x * CH;
   double k[9];
 #pragma unroll
   for (int x = 0; x < 9; ++x) k[x] = B.v(F_DXIDX, x + 1, n);
@@ -211,57 +240,74 @@ __global__ void k_pipe_recs(const BlockView* __restrict__ blocks, CaseConsts cc_
     rec[PW_DIR / 2 + 3 * d] = double2{uu, x};
     rec[PW_DIR / 2 + 3 * d + 1] = double2{y, z};
     rec[PW_DIR / 2 + 3 * d + 2] = double2{rad, hj};
-    B.s(F_RA + d, n) = rad;
+    if (act) B.s(F_RA + d, n) = rad;
   }
   rec[PW_M / 2] = double2{mu, mv};
   rec[PW_M / 2 + 1] = double2{mw, rho};
   rec[PW_RCP / 2] = double2{fast ? rrho : __longlong_as_double(0x7ff8000000000000ll), recip_lo(rho, rrho)};
   rec[PW_PHI / 2] = double2{phi, a1};
+  store_records<CH>(sm + (threadIdx.x & ~31u) * CH, B.pipe.rec, kPipeRec, 0, p, -1);
 }
 
 // rhs = rhsi + rhsv and the diagonal phi/dt + ra + rb + rc of every updated
 // node (sub_timeadvancement_1stimplicit.f90:72-156; 2-D: no zeta radius), rhs in
-// its place of the box too (the residual norm reads it there).
+// its place of the box too (the residual norm reads it there).  Plate: 73 us, 89
+// with each thread storing its own record.
 __global__ void k_pipe_sca(const BlockView* __restrict__ blocks, CaseConsts cc_launch) {
   const BlockView& B = blocks[blockIdx.y];
   if (B.retired()) return;
   const CaseConsts& cc = B.ccb ? *B.ccb : cc_launch;
   const int u = (int)(blockIdx.x * blockDim.x + threadIdx.x);
-  if (u >= B.b1.size()) return;
-  const long n = box_node(B, u);
-  double* rec = B.pipe.rec + (long)kPipeRec * B.pipe.at[u];
-  double2* rec2 = reinterpret_cast<double2*>(rec);
-  double r[5];
+  if (u - (int)threadIdx.x >= B.b1.size()) return;  // the whole CTA
+  constexpr int CH = (PW_OK + 1 - PW_DIV) / 2;
+  __shared__ double2 sm[128 * CH];
+  const bool act = u < B.b1.size();
+  const long n = box_node(B, act ? u : 0);
+  const int p = act ? B.pipe.at[u] : -1;
+  double2* rec = sm + threadIdx.x * CH;
+  // every load before the first store and division, so that all are in flight at once
+  const double dt = B.s(F_DT, n), ra = B.s(F_RA, n), rb = B.s(F_RB, n), rc = B.s(F_RC, n), invj = B.s(F_INVJ, n);
+  double ri5[5], r[5];
 #pragma unroll
   for (int c = 0; c < 5; ++c) {
-    r[c] = B.v(F_RHSI, c + 1, n) + B.v(F_RHSV, c + 1, n);
-    B.v(F_RHS, c + 1, n) = r[c];
+    ri5[c] = B.v(F_RHSI, c + 1, n);
+    r[c] = B.v(F_RHSV, c + 1, n);
+  }
+#pragma unroll
+  for (int c = 0; c < 5; ++c) {
+    r[c] = ri5[c] + r[c];
+    if (act) B.v(F_RHS, c + 1, n) = r[c];
   }
   const double phi = cc.cfl >= 1.0e3 ? 0.0 : 1.0;
-  double diag = phi * 1.0 / B.s(F_DT, n) + B.s(F_RA, n) + B.s(F_RB, n);
-  if (!B.planar()) diag = diag + B.s(F_RC, n);
-  const double invj = B.s(F_INVJ, n);
+  double diag = phi * 1.0 / dt + ra + rb;
+  if (!B.planar()) diag = diag + rc;
   const double rd = 1.0 / diag, ri = 1.0 / invj;
-  rec2[PW_DIV / 2] = double2{diag, invj};
-  rec2[PW_DIV / 2 + 1] = double2{rd, ri};
-  rec2[PW_DIV / 2 + 2] = double2{recip_lo(diag, rd), recip_lo(invj, ri)};
-  rec2[PW_RHS / 2] = double2{r[0], r[1]};
-  rec2[PW_RHS / 2 + 1] = double2{r[2], r[3]};
-  rec2[PW_RHS / 2 + 2] = double2{r[4], divisors_ok(diag, invj) ? 1.0 : 0.0};
+  rec[0] = double2{diag, invj};
+  rec[1] = double2{rd, ri};
+  rec[2] = double2{recip_lo(diag, rd), recip_lo(invj, ri)};
+  rec[3] = double2{r[0], r[1]};
+  rec[4] = double2{r[2], r[3]};
+  rec[5] = double2{r[4], divisors_ok(diag, invj) ? 1.0 : 0.0};
+  store_records<CH>(sm + (threadIdx.x & ~31u) * CH, B.pipe.rec, kPipeRec, PW_DIV, p, -1);
 }
 
 // The SA sweeps' records (sub_tur_sa.f90:676-750, :762-778): the upwind
 // coefficients 0.5*(U + |U|) and 0.5*(U - |U|) per direction, sa_rhs and the
-// diagonal.
+// diagonal.  Plate: 57 us, 78 with each thread storing its own record.
 __global__ void k_pipe_sa_recs(const BlockView* __restrict__ blocks, CaseConsts cc_launch) {
   const BlockView& B = blocks[blockIdx.y];
   if (B.retired()) return;
   const CaseConsts& cc = B.ccb ? *B.ccb : cc_launch;
-  const int p = (int)(blockIdx.x * blockDim.x + threadIdx.x);
-  if (p >= B.b1.size()) return;
-  const long n = box_node(B, p);
+  const int u0 = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+  if (u0 - (int)threadIdx.x >= B.b1.size()) return;  // the whole CTA
+  constexpr int CH = kPipeSaRec / 2;
+  __shared__ double2 sm[128 * CH];
+  const bool act = u0 < B.b1.size();
+  const long n = box_node(B, act ? u0 : 0);
+  const int p = act ? B.pipe.at[u0] : -1;
   const double phi = (cc.cfl >= 1.0e3 && cc.time == IFLAG_STEADY) ? 0.0 : 1.0;
   const double u = B.v(F_PRI, 2, n), v = B.v(F_PRI, 3, n), w = B.v(F_PRI, 4, n), nut = B.s(F_NUT, n);
+  const double dt = B.s(F_DT, n), diasd = B.s(F_DIASD, n), rhs = B.s(F_SARHS, n);
   double c[3], d2 = 0.0;
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
@@ -270,17 +316,18 @@ __global__ void k_pipe_sa_recs(const BlockView* __restrict__ blocks, CaseConsts 
     c[d] = x * u + y * v + z * w;
   }
   const double tm = 4.0 * d2 * nut / cc.re;
-  const double diag = 1.0 / B.s(F_DT, n) * phi + fabs(c[0]) + fabs(c[1]) + fabs(c[2]) + tm - B.s(F_DIASD, n);
+  const double diag = 1.0 / dt * phi + fabs(c[0]) + fabs(c[1]) + fabs(c[2]) + tm - diasd;
   const double rd = 1.0 / diag;
-  double* rec = B.pipe.sa_rec + (long)kPipeSaRec * B.pipe.at[p];
-  double2* rec2 = reinterpret_cast<double2*>(rec);
+  double2* rec2 = sm + threadIdx.x * CH;
   rec2[SW_A / 2] = double2{0.5 * (c[0] + fabs(c[0])), 0.5 * (c[1] + fabs(c[1]))};
-  rec[SW_A + 2] = 0.5 * (c[2] + fabs(c[2]));
+  rec2[SW_A / 2 + 1] = double2{0.5 * (c[2] + fabs(c[2])), 0.0};
   rec2[SW_B / 2] = double2{0.5 * (c[0] - fabs(c[0])), 0.5 * (c[1] - fabs(c[1]))};
   rec2[SW_B / 2 + 1] = double2{0.5 * (c[2] - fabs(c[2])), __longlong_as_double((long long)n)};
-  rec2[SW_RHS / 2] = double2{B.s(F_SARHS, n), diag};
+  rec2[SW_RHS / 2] = double2{rhs, diag};
   rec2[SW_RHS / 2 + 1] = double2{rd, recip_lo(diag, rd)};
   rec2[SW_NUT / 2] = double2{nut, divisors_ok(diag, 1.0) ? 1.0 : 0.0};
+  // (the neighbour word beside the third coefficient stays)
+  store_records<CH>(sm + (threadIdx.x & ~31u) * CH, B.pipe.sa_rec, kPipeSaRec, 0, p, SW_NBR / 2);
 }
 
 // q += dq over the updated box (sub_timeadvancement_1stimplicit.f90:568-574), in
@@ -297,7 +344,6 @@ __global__ void k_pipe_update(const BlockView* __restrict__ blocks) {
 }
 
 // ------------------------------------------------------------------ the sweeps
-#ifdef __CUDACC__  // (the order's tables above also build as host code, for their test)
 namespace {
 
 // The 25 entries of calc_jm's A with rs on the diagonal, times hj, by IEEE
