@@ -1075,7 +1075,10 @@ __device__ __forceinline__ void lusgs_bulk_body(const BlockView* __restrict__ bl
   };
   auto slice_bytes = [&](int cnt, unsigned r) -> unsigned {
     const int n = min(T, 5 * cnt - (int)r * T);
-    return n <= 0 ? 0u : (unsigned)((n * 8 + 15) & ~15);
+    // a CTA without items sends 16 unread bytes (its place in the ring is free),
+    // so that no CTA gets two planes ahead of one that holds none of them: a
+    // phase that counts two planes' bytes would never complete
+    return n <= 0 ? 16u : (unsigned)((n * 8 + 15) & ~15);
   };
   // this thread's row of the next DEPTH planes, loaded ahead (records and
   // scalars are read-only during the sweep)
