@@ -540,24 +540,27 @@ PipeFit pipe_fit(const BlockView* hv, int nblk, int C) {
     cuts = std::max(cuts, t.ce);
   }
   if (P > 1022) return f;  // the neighbour words' index range
-  // one CTA of up to 16 warps per SM or, where the clusters outnumber the SMs,
-  // two of up to 8
-  const bool two = nblk * C > kSms;
-  const int most = two ? 7 : 15;  // compute warps
-  const size_t limit = (size_t)(two ? 113 : 226) * 1024;
   PipeShape& s = f.sh;
   s.P = P;
   s.L = L;
-  s.W = std::min(most, (P + 9) / 10);
-  // up to seven groups while the CTA keeps to 8 warps (200 registers each),
-  // else two within 11 (168 registers)
-  s.NG = s.W <= 3 ? 7 / s.W : (!two && s.W <= 5) ? 2 : 1;
-  s.NST = s.NG + 3;
-  s.D = 8;
   auto bytes = [&] { return (size_t)PipeSmem(s, kPipeRec, kPipeProd, 5, H).words * sizeof(double); };
-  while (bytes() > limit && s.NST > std::max(2, s.NG)) --s.NST;
-  while (bytes() > limit && s.NG > 1) s.NST = std::max(2, --s.NG);
-  if (bytes() > limit) return f;
+  // one CTA of up to 16 warps per SM or, where the clusters outnumber the SMs
+  // and two stages of a plane fit half of one, two of up to 8
+  bool two = nblk * C > kSms;
+  size_t limit = 0;
+  for (;; two = false) {
+    limit = (size_t)(two ? 113 : 226) * 1024;
+    s.W = std::min(two ? 7 : 15, (P + 9) / 10);  // compute warps
+    // up to seven groups while the CTA keeps to 8 warps (200 registers each),
+    // else two within 11 (168 registers)
+    s.NG = s.W <= 3 ? 7 / s.W : (!two && s.W <= 5) ? 2 : 1;
+    s.NST = s.NG + 3;
+    s.D = 8;
+    while (bytes() > limit && s.NST > std::max(2, s.NG)) --s.NST;
+    while (bytes() > limit && s.NG > 1) s.NST = std::max(2, --s.NG);
+    if (bytes() <= limit) break;
+    if (!two) return f;
+  }
   // more messages on the way while three quarters of that hold them
   while (s.D < 64 && (s.D *= 2, bytes() <= limit / 4 * 3)) {
   }

@@ -3,6 +3,8 @@ field (the arithmetic is the oracle's), for block shapes at the edges of the
 cuts: a single updated node, extents below the cluster's size, planes wider than
 a CTA's warps, many blocks (two CTAs per SM), one layer per slab, planes too wide
 for the pipeline, and mixed precision against FP64."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -81,3 +83,29 @@ def test_planes_too_wide_for_the_pipeline(gpu):
         finally:
             gc.close()
     assert relerr(q[True], q[False]) <= 1e-6
+
+
+def test_wide_blocks_outnumbering_the_sms(gpu):
+    """Clusters of more CTAs than the device has SMs whose planes leave no room
+    for a second CTA per SM: the sweeps through global memory give the same bits."""
+    q = []
+    for piped in (True, False):
+        case = channels(20, 42, 42, 42)()
+        gc = gpu.GpuCase(case)
+        try:
+            if not piped:
+                gc.set_sweep_cluster(1)
+            gc.compute_geometry()
+            gc.init_flowfield()
+            gc.start()
+            gc.step(2)
+            gc.sync_to_host(gpu.mask("q"))
+            assert gc.status() == 0
+            gc.set_register_bound(False)  # (writes the shapes' text)
+            gc.L.aero_tuning.restype = ctypes.c_char_p
+            assert ("pipelined" in gc.L.aero_tuning().decode()) == piped
+            q.append([b.fields["q"].copy() for b in case.blocks])
+        finally:
+            gc.close()
+    for a, b in zip(*q):
+        assert np.all(np.isfinite(a)) and np.array_equal(a, b)
