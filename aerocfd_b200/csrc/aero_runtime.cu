@@ -1259,11 +1259,6 @@ int do_getpri_all() {
   return launch_getpri(g.d_blocks, (int)g.blocks.size(), g.max_box, g.cc);
 }
 
-// One iteration of main.f90:343-447 over every block.  main.f90:446 recomputes
-// the primitives at the end of an iteration from the same q that :357 uses at
-// the start of the next one, so the device computes them once, at the start;
-// aero_step recomputes them after its last iteration so the state it leaves
-// matches the reference's.
 // crank2nd on nblk views (sub_timeadvancement_2ndcrank.f90): dual-time rhs,
 // dq = 0, the i, j, k line recurrences, q += dq/inv_j.
 int launch_crank(const BlockView* views, int nblk, long maxN, long maxN1, const Box* lines, const CaseConsts& cc) {
@@ -1349,12 +1344,24 @@ int do_retire() {
   return AERO_OK;
 }
 
+// One iteration of main.f90:343-447 over every block.  main.f90:446 recomputes
+// the primitives at the end of an iteration from the same q that :357 uses at
+// the start of the next one, so the steps of one call compute them once per
+// iteration, at its end (where a block that has failed is marked before the
+// next step's k_retire), and before the first (opening_primitives): one pass
+// over the boxes less per step, 25 of the plate's 1350 us.
+int opening_primitives() {
+  int rc;
+  if (crank_on()) return AERO_OK;  // (each of its sub-iterations computes them)
+  if ((rc = do_retire())) return rc;
+  return do_getpri_all();
+}
+
 int do_iteration(bool want_dt_minmax, bool resid_beside = false) {
   int rc;
   if ((rc = do_retire())) return rc;
   if (crank_on()) return do_iteration_crank();
   int nb = (int)g.blocks.size();
-  if ((rc = do_getpri_all())) return rc;
   // inviscid_flux_1 (rhsi and its face scratch) beside viscous_flux and
   // find_dt (rhsv, amu, vor, dudx, tao, their scratch, dt): neither side reads
   // what the other writes
@@ -1436,7 +1443,8 @@ CaseConsts consts_from(const int* iflags, const double* params) {
   return c;
 }
 
-// One time step as aero_step runs it: the iteration, the closing primitives
+// One time step as aero_step runs it, the primitives at hand (opening_primitives
+// or the step before): the iteration, the closing primitives
 // and the residual norm (into g.d_out; beside the sweeps for the implicit
 // update, after the step for the dual-time one).
 int step_once() {
@@ -1789,6 +1797,7 @@ int aero_autotune(int iters) {
   CK(cudaEventCreate(&b));
   auto time_steps = [&](double& ms) -> int {
     int r;
+    if ((r = opening_primitives())) return r;
     if ((r = step_once())) return r;  // warm
     CK(cudaEventRecord(a, g.stream));
     for (int x = 0; x < iters; ++x)
@@ -2951,6 +2960,7 @@ int aero_step_timed(int nsteps, int flush_l2, double* device_ms) {
   for (int s = 0; s < nsteps; ++s) {
     if (flush_l2) CK(cudaMemsetAsync(flush, s & 0xff, fbytes, g.stream));
     CK(cudaEventRecord(a, g.stream));
+    if ((rc = opening_primitives())) return rc;
     if ((rc = run_step())) return rc;  // iteration, closing primitives, residual
     CK(cudaEventRecord(b, g.stream));
     CK(cudaEventSynchronize(b));
@@ -3010,6 +3020,7 @@ int aero_launch_count(unsigned long long* count) {
 int aero_step(int nsteps, double* resid_hist, double* dt_minmax) {
   int rc = need_setup();
   if (rc) return rc;
+  if (nsteps > 0 && (rc = opening_primitives())) return rc;
   // The residuals of up to kHistSteps steps cross the bus into pinned memory
   // behind their steps; the host waits once per that many steps, so that it
   // launches the next step while the device runs this one.

@@ -109,3 +109,32 @@ def test_wide_blocks_outnumbering_the_sms(gpu):
             gc.close()
     for a, b in zip(*q):
         assert np.all(np.isfinite(a)) and np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("graphs", [False, True])
+def test_steps_of_one_call_and_of_several(gpu, graphs):
+    """The primitives that open a step are the ones that closed the step before:
+    three steps in one call, or one by one, or after a field that went to the
+    device between two calls, are the same."""
+    out = []
+    for split in ([3], [1, 1, 1], [2, 1]):
+        case = plate(1, 1, 1, ni=17, nj=13, nk=7)()
+        gc = gpu.GpuCase(case)
+        try:
+            gc.use_graphs(graphs)
+            gc.compute_geometry()
+            gc.init_flowfield()
+            gc.start()
+            h = []
+            for n in split:
+                gc.sync_to_host(gpu.mask("q", "nut"))
+                gc.sync_to_device(gpu.mask("q", "nut"))
+                h.append(gc.step(n))
+            gc.sync_to_host(gpu.mask("q", "nut", "pri_v"))
+            b = case.blocks[0].fields
+            out.append([np.concatenate(h)] + [b[k].copy() for k in ("q", "nut", "pri_v")])
+        finally:
+            gc.close()
+    for o in out[1:]:
+        for a, b in zip(out[0], o):
+            assert np.array_equal(a, b)
