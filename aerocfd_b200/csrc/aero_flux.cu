@@ -854,13 +854,8 @@ __global__ void k_fill(const BlockView* __restrict__ blocks, int fid, int nc, do
 }
 
 // --------------------------------------------------------------- viscous flux
-// Central difference along one direction inside the physical range, one-sided
-// at its ends (sub_viscous.f90:106-178 and :296-340).
-__device__ __forceinline__ double cdiff(const double* f, long n, long st, int pos, int lo, int hi) {
-  if (pos == lo) return f[n + st] - f[n];
-  if (pos == hi) return f[n] - f[n - st];
-  return (f[n + st] - f[n - st]) / 2.0;
-}
+// (central differences inside the physical range, one-sided at its ends:
+// sub_viscous.f90:106-178 and :296-340)
 
 // sub_viscous.f90:187-293: gradients, Sutherland viscosity, stresses, heat flux,
 // vorticity and the contravariant viscous fluxes on the physical nodes.  The
@@ -885,24 +880,26 @@ __device__ __forceinline__ void viscous_a_body(const BlockView* __restrict__ blo
   const double* pv = B.f[F_PRI] + 2 * B.plane;
   const double* pw = B.f[F_PRI] + 3 * B.plane;
   const double* pt = B.f[F_PRI] + 5 * B.plane;
-  double gt[3] = {0, 0, 0}, gu[3] = {0, 0, 0}, gv[3] = {0, 0, 0}, gw[3] = {0, 0, 0};
-  int ndir = cc.dimension == IFLAG_3D ? 3 : 2;
-  for (int d = 0; d < ndir; ++d) {
-    gt[d] = cdiff(pt, n, st[d], pos[d], lo[d], hi[d]);
-    gu[d] = cdiff(pu, n, st[d], pos[d], lo[d], hi[d]);
-    gv[d] = cdiff(pv, n, st[d], pos[d], lo[d], hi[d]);
-    gw[d] = cdiff(pw, n, st[d], pos[d], lo[d], hi[d]);
+  double gt[3], gu[3], gv[3], gw[3];
+  // (every load comes before the first store)
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    const NodeDiff D(n, st[d], pos[d], lo[d], hi[d], d < 2 || cc.dimension == IFLAG_3D);
+    gt[d] = D(pt);
+    gu[d] = D(pu);
+    gv[d] = D(pv);
+    gw[d] = D(pw);
   }
   double u0 = pu[n], v0 = pv[n], w0 = pw[n], t0 = pt[n];
+  double amu2 = B.v(F_AMU, 2, n), ij = B.s(F_INVJ, n);
+  double m[9];
+#pragma unroll
+  for (int c = 0; c < 9; ++c) m[c] = B.v(F_DXIDX, c + 1, n);
   double amu1 = (1.0 + 124.0 / cc.tinf) / (t0 + 124.0 / cc.tinf) * crm::pow(t0, 1.5);
-  double amu2 = B.v(F_AMU, 2, n);
   double amu3 = amu1 + amu2;
   B.v(F_AMU, 1, n) = amu1;
   B.v(F_AMU, 3, n) = amu3;
   double ki = cc.gamma * cc.cv * (amu1 / cc.prl + amu2 / cc.prt);
-  double m[9];
-#pragma unroll
-  for (int c = 0; c < 9; ++c) m[c] = B.v(F_DXIDX, c + 1, n);
   double tx = gt[0] * m[0] + gt[1] * m[3] + gt[2] * m[6];
   double ty = gt[0] * m[1] + gt[1] * m[4] + gt[2] * m[7];
   double tz = gt[0] * m[2] + gt[1] * m[5] + gt[2] * m[8];
@@ -929,7 +926,6 @@ __device__ __forceinline__ void viscous_a_body(const BlockView* __restrict__ blo
 #pragma unroll
     for (int c = 0; c < 6; ++c) B.v(F_TAO, c + 1, n) = ta[c];
   }
-  double ij = B.s(F_INVJ, n);
   double* fvh = B.f[F_FVH];
   long P = B.plane;
   // fv/gv/hv components 2..5 -> FVH planes 0..3 (fv), 4..7 (gv), 8..11 (hv)
@@ -978,26 +974,27 @@ __global__ void k_viscous_a_mixed(const BlockView* __restrict__ blocks, CaseCons
   const double* pv = B.f[F_PRI] + 2 * B.plane;
   const double* pw = B.f[F_PRI] + 3 * B.plane;
   const double* pt = B.f[F_PRI] + 5 * B.plane;
-  float gt[3] = {0, 0, 0}, gu[3] = {0, 0, 0}, gv[3] = {0, 0, 0}, gw[3] = {0, 0, 0};
-  int ndir = cc.dimension == IFLAG_3D ? 3 : 2;
-  for (int d = 0; d < ndir; ++d) {
-    gt[d] = (float)cdiff(pt, n, st[d], pos[d], lo[d], hi[d]);
-    gu[d] = (float)cdiff(pu, n, st[d], pos[d], lo[d], hi[d]);
-    gv[d] = (float)cdiff(pv, n, st[d], pos[d], lo[d], hi[d]);
-    gw[d] = (float)cdiff(pw, n, st[d], pos[d], lo[d], hi[d]);
+  float gt[3], gu[3], gv[3], gw[3];
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    const NodeDiff D(n, st[d], pos[d], lo[d], hi[d], d < 2 || cc.dimension == IFLAG_3D);
+    gt[d] = (float)D(pt);
+    gu[d] = (float)D(pu);
+    gv[d] = (float)D(pv);
+    gw[d] = (float)D(pw);
   }
   double t0 = pt[n];
-  double amu1 = (1.0 + 124.0 / cc.tinf) / (t0 + 124.0 / cc.tinf) * crm::pow(t0, 1.5);
   double amu2 = B.v(F_AMU, 2, n);
+  float u0 = (float)pu[n], v0 = (float)pv[n], w0 = (float)pw[n], ij = (float)B.s(F_INVJ, n);
+  float m[9];
+#pragma unroll
+  for (int c = 0; c < 9; ++c) m[c] = (float)B.v(F_DXIDX, c + 1, n);
+  double amu1 = (1.0 + 124.0 / cc.tinf) / (t0 + 124.0 / cc.tinf) * crm::pow(t0, 1.5);
   double amu3d = amu1 + amu2;
   B.v(F_AMU, 1, n) = amu1;
   B.v(F_AMU, 3, n) = amu3d;
   float amu3 = (float)amu3d;
   float ki = (float)(cc.gamma * cc.cv * (amu1 / cc.prl + amu2 / cc.prt));
-  float u0 = (float)pu[n], v0 = (float)pv[n], w0 = (float)pw[n];
-  float m[9];
-#pragma unroll
-  for (int c = 0; c < 9; ++c) m[c] = (float)B.v(F_DXIDX, c + 1, n);
   float tx = gt[0] * m[0] + gt[1] * m[3] + gt[2] * m[6];
   float ty = gt[0] * m[1] + gt[1] * m[4] + gt[2] * m[7];
   float tz = gt[0] * m[2] + gt[1] * m[5] + gt[2] * m[8];
@@ -1025,7 +1022,6 @@ __global__ void k_viscous_a_mixed(const BlockView* __restrict__ blocks, CaseCons
 #pragma unroll
     for (int c = 0; c < 6; ++c) B.v(F_TAO, c + 1, n) = (double)ta[c];
   }
-  float ij = (float)B.s(F_INVJ, n);
   double* fvh = B.f[F_FVH];
   long P = B.plane;
 #pragma unroll
@@ -1057,15 +1053,14 @@ __global__ void k_viscous_b(const BlockView* __restrict__ blocks, CaseConsts cc_
   const int hi[3] = {b0.ie, b0.je, b0.ke};
   const double* fvh = B.f[F_FVH];
   long P = B.plane;
-  bool three = cc.dimension == IFLAG_3D;
+  const NodeDiff A(n, st[0], pos[0], lo[0], hi[0]), E(n, st[1], pos[1], lo[1], hi[1]);
+  const NodeDiff Z(n, st[2], pos[2], lo[2], hi[2], cc.dimension == IFLAG_3D);
+  double sum[4];
+#pragma unroll
+  for (int c = 0; c < 4; ++c) sum[c] = A(fvh + c * P) + E(fvh + (4 + c) * P) + Z(fvh + (8 + c) * P);
   B.v(F_RHSV, 1, n) = 0.0;  // fv(1)=gv(1)=hv(1)=0: ((0+0)+0)/re
 #pragma unroll
-  for (int c = 0; c < 4; ++c) {
-    double a = cdiff(fvh + (0 + c) * P, n, st[0], pos[0], lo[0], hi[0]);
-    double b = cdiff(fvh + (4 + c) * P, n, st[1], pos[1], lo[1], hi[1]);
-    double h = three ? cdiff(fvh + (8 + c) * P, n, st[2], pos[2], lo[2], hi[2]) : 0.0;
-    B.v(F_RHSV, c + 2, n) = (a + b + h) / cc.re;
-  }
+  for (int c = 0; c < 4; ++c) B.v(F_RHSV, c + 2, n) = sum[c] / cc.re;
 }
 
 // ------------------------------------------------------------------ time step

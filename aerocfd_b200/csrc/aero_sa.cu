@@ -15,13 +15,6 @@ namespace aero {
 
 namespace {
 
-// One-sided at the physical ends is0/ie0, central elsewhere (sub_tur_sa.f90:297-303).
-__device__ __forceinline__ double d1(const double* f, long n, long st, int pos, int lo0, int hi0) {
-  if (pos == lo0) return f[n + st] - f[n];
-  if (pos == hi0) return f[n] - f[n - st];
-  return (f[n + st] - f[n - st]) / 2.0;
-}
-
 __device__ __forceinline__ void node_of(const Box& bx, long t, int& i, int& j, int& k) {
   i = bx.is + (int)(t % bx.nx());
   long r = t / bx.nx();
@@ -48,19 +41,27 @@ __global__ void k_sa_a(const BlockView* __restrict__ blocks, CaseConsts cc_launc
   const int pos[3] = {i, j, k};
   const int lo0[3] = {B.b0.is, B.b0.js, B.b0.ks}, hi0[3] = {B.b0.ie, B.b0.je, B.b0.ke};
   const double* nut = B.f[F_NUT];
-  double g[3] = {0.0, 0.0, 0.0};
-  int ndir = cc.dimension == IFLAG_3D ? 3 : 2;
-  for (int d = 0; d < ndir; ++d) g[d] = d1(nut, n, st[d], pos[d], lo0[d], hi0[d]);
+  // one-sided at the physical ends is0/ie0, central elsewhere (sub_tur_sa.f90:297-303);
+  // every load comes before the first store
+  double g[3], con[3];
+#pragma unroll
+  for (int d = 0; d < 3; ++d)
+    g[d] = NodeDiff(n, st[d], pos[d], lo0[d], hi0[d], d < 2 || cc.dimension == IFLAG_3D)(nut);
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    const int f = d == 0 ? F_ALPHA : d == 1 ? F_BETA : F_GAMMA;
+    con[d] = B.v(f, 1, n) * g[0] + B.v(f, 2, n) * g[1] + B.v(f, 3, n) * g[2];
+  }
+  const double amu = B.v(F_AMU, 1, n), rho = B.v(F_PRI, 1, n), nut0 = nut[n];
   double* S = B.f[F_SAS];
   long P = B.plane;
-  S[0 * P + n] = g[0];
-  S[1 * P + n] = g[1];
-  S[2 * P + n] = g[2];
-  S[3 * P + n] = B.v(F_ALPHA, 1, n) * g[0] + B.v(F_ALPHA, 2, n) * g[1] + B.v(F_ALPHA, 3, n) * g[2];
-  S[4 * P + n] = B.v(F_BETA, 1, n) * g[0] + B.v(F_BETA, 2, n) * g[1] + B.v(F_BETA, 3, n) * g[2];
-  S[5 * P + n] = B.v(F_GAMMA, 1, n) * g[0] + B.v(F_GAMMA, 2, n) * g[1] + B.v(F_GAMMA, 3, n) * g[2];
-  double nu0 = B.v(F_AMU, 1, n) / B.v(F_PRI, 1, n);
-  S[6 * P + n] = nu0 + (1.0 + SA_CB2) * nut[n];
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    S[d * P + n] = g[d];
+    S[(3 + d) * P + n] = con[d];
+  }
+  double nu0 = amu / rho;
+  S[6 * P + n] = nu0 + (1.0 + SA_CB2) * nut0;
 }
 
 // Pass B over the updated box: sa_rhs = advection (sa_rhs1) + diffusion
@@ -90,20 +91,21 @@ __device__ __forceinline__ void sa_b_body(const BlockView* __restrict__ blocks, 
   double u = B.v(F_PRI, 2, n), v = B.v(F_PRI, 3, n), w = B.v(F_PRI, 4, n);
   double nut0 = nut[n];
   // sa_rhs1: first-order upwind advection on the contravariant velocities
-  double adv[3] = {0.0, 0.0, 0.0};
-  for (int d = 0; d < (three ? 3 : 2); ++d) {
+  double adv[3];
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    const bool on = d < 2 || three;
     double uu = m[3 * d] * u + m[3 * d + 1] * v + m[3 * d + 2] * w;
-    double nutp = nut[n + st[d]], nutm = nut[n - st[d]];
-    adv[d] = -(0.5 * (uu + fabs(uu)) * (nut0 - nutm) + 0.5 * (uu - fabs(uu)) * (nutp - nut0));
+    double nutp = nut[on ? n + st[d] : n], nutm = nut[on ? n - st[d] : n];
+    const double a = -(0.5 * (uu + fabs(uu)) * (nut0 - nutm) + 0.5 * (uu - fabs(uu)) * (nutp - nut0));
+    adv[d] = on ? a : 0.0;
   }
   double rhs = adv[0] + adv[1] + adv[2];
   // sa_rhs2: diffusion
-  double ta = d1(S + 3 * P, n, st[0], pos[0], lo0[0], hi0[0]);
-  double tb = d1(S + 4 * P, n, st[1], pos[1], lo0[1], hi0[1]);
-  double tc = three ? d1(S + 5 * P, n, st[2], pos[2], lo0[2], hi0[2]) : 0.0;
-  double txi = d1(S + 6 * P, n, st[0], pos[0], lo0[0], hi0[0]);
-  double teta = d1(S + 6 * P, n, st[1], pos[1], lo0[1], hi0[1]);
-  double tzeta = three ? d1(S + 6 * P, n, st[2], pos[2], lo0[2], hi0[2]) : 0.0;
+  const NodeDiff A(n, st[0], pos[0], lo0[0], hi0[0]), E(n, st[1], pos[1], lo0[1], hi0[1]);
+  const NodeDiff Z(n, st[2], pos[2], lo0[2], hi0[2], three);
+  double ta = A(S + 3 * P), tb = E(S + 4 * P), tc = Z(S + 5 * P);
+  double txi = A(S + 6 * P), teta = E(S + 6 * P), tzeta = Z(S + 6 * P);
   double tx = txi * m[0] + teta * m[3] + tzeta * m[6];
   double ty = txi * m[1] + teta * m[4] + tzeta * m[7];
   double tz = txi * m[2] + teta * m[5] + tzeta * m[8];
@@ -196,20 +198,21 @@ __global__ void k_sa_b_mixed(const BlockView* __restrict__ blocks, CaseConsts cc
   const double nut0d = nut[n];
   const float nut0 = (float)nut0d;
   // sa_rhs1: first-order upwind advection
-  float adv[3] = {0.0f, 0.0f, 0.0f};
-  for (int d = 0; d < (three ? 3 : 2); ++d) {
+  float adv[3];
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    const bool on = d < 2 || three;
     float uu = m[3 * d] * u + m[3 * d + 1] * v + m[3 * d + 2] * w;
-    float dm = (float)(nut0d - nut[n - st[d]]), dp = (float)(nut[n + st[d]] - nut0d);
-    adv[d] = -(0.5f * (uu + fabsf(uu)) * dm + 0.5f * (uu - fabsf(uu)) * dp);
+    float dm = (float)(nut0d - nut[on ? n - st[d] : n]), dp = (float)(nut[on ? n + st[d] : n] - nut0d);
+    const float a = -(0.5f * (uu + fabsf(uu)) * dm + 0.5f * (uu - fabsf(uu)) * dp);
+    adv[d] = on ? a : 0.0f;
   }
   double rhs = (double)adv[0] + (double)adv[1] + (double)adv[2];
   // sa_rhs2: diffusion
-  float ta = (float)d1(S + 3 * P, n, st[0], pos[0], lo0[0], hi0[0]);
-  float tb = (float)d1(S + 4 * P, n, st[1], pos[1], lo0[1], hi0[1]);
-  float tc = three ? (float)d1(S + 5 * P, n, st[2], pos[2], lo0[2], hi0[2]) : 0.0f;
-  float txi = (float)d1(S + 6 * P, n, st[0], pos[0], lo0[0], hi0[0]);
-  float teta = (float)d1(S + 6 * P, n, st[1], pos[1], lo0[1], hi0[1]);
-  float tzeta = three ? (float)d1(S + 6 * P, n, st[2], pos[2], lo0[2], hi0[2]) : 0.0f;
+  const NodeDiff A(n, st[0], pos[0], lo0[0], hi0[0]), E(n, st[1], pos[1], lo0[1], hi0[1]);
+  const NodeDiff Z(n, st[2], pos[2], lo0[2], hi0[2], three);
+  float ta = (float)A(S + 3 * P), tb = (float)E(S + 4 * P), tc = (float)Z(S + 5 * P);
+  float txi = (float)A(S + 6 * P), teta = (float)E(S + 6 * P), tzeta = (float)Z(S + 6 * P);
   float tx = txi * m[0] + teta * m[3] + tzeta * m[6];
   float ty = txi * m[1] + teta * m[4] + tzeta * m[7];
   float tz = txi * m[2] + teta * m[5] + tzeta * m[8];
