@@ -90,8 +90,8 @@ const char* aero_last_error(void);
 int aero_get_status(unsigned* status);
 /* Where the first cluster-sweep wait that gave up (AERO_ST_TIMEOUT) was, since
  * the last call: out5 = sweep (1: mean-flow bulk exchange, 2: mean-flow slab,
- * 3: SA slab, 4: the one-CTA staged sweep, whose waits have the poll budget
- * of aero_set_poll_budget), block (0-based), the CTA's rank in its cluster, the step
+ * 3: SA, pipelined or slab, 4: the pipelined mean-flow sweep or the one-CTA
+ * staged one, whose waits have the poll budget of aero_set_poll_budget), block (0-based), the CTA's rank in its cluster, the step
  * (plane step of the forward then backward pass) and the wait (1: a plane's
  * values, 2: the downstream slab's progress, 3: the last plane's values);
  * all -1 when none gave up.  Clears the record.  The cluster sweeps bound
@@ -350,8 +350,10 @@ const char* aero_tuning(void);
  * the mixed face kernel bounded for 10), 32, 64 or 128; element-wise threads 128, 256,
  * 512; viscous and block-record threads 64, 128, 256; sweep stages 2..4. */
 int aero_set_tuning(int inv_tile, int ew, int visc, int mats, int nst_max);
-/* CTAs that share each block's LU-SGS sweep: 1 (one CTA per block, the
- * records staged in shared memory when its planes fit) or a thread-block
+/* By default each block's LU-SGS sweeps run as a pipeline of slabs over a
+ * cluster whose size a rule or the autotuner chooses, where the planes fit.
+ * This call selects another sweep instead, by the CTAs that share a block: 1
+ * (one CTA per block, the records staged in shared memory when its planes fit) or a thread-block
  * cluster of 2, 4 or 8 CTAs, or 16 CTAs (a non-portable cluster size, with
  * the bulk-copy or the slab exchange only; accepted after aero_finish_setup
  * when the device can hold such a cluster).  The arithmetic is the same for
@@ -368,7 +370,7 @@ int aero_set_sweep_cluster(int ctas);
  * built for two resident per SM (for batches whose sweep CTAs outnumber the
  * SMs; larger CTAs take 1).  The arithmetic is the same for every choice. */
 int aero_set_sweep_exchange(int mode);
-/* CTAs that share each block's SA sweep: 1 (default; one CTA per block) or a
+/* The same for the SA sweep: 1 (one CTA per block) or a
  * cluster of 2, 4 or 8 CTAs pipelined by k-slabs as exchange 2 above (used
  * when each slab's part of a plane has at most 512 nodes), or 16 (accepted
  * after aero_finish_setup when the device can hold such a cluster).  The
