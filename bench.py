@@ -79,8 +79,8 @@ KERNEL_BOX = {"k_lusgs_sweep": "box1", "k_inviscid": "box1", "k_viscous_a": "box
               "k_residual_partial": "box1", "k_lusgs_mats": "box1", "k_sa_sweep": "box1", "k_sa_a": "box1"}
 # DRAM bytes (read + write) per launch of the dominant kernel of each
 # workload, from one ncu capture of it (cold cache under replay).
-KERNEL_TRAFFIC = {(WORKLOAD, "k_lusgs_sweep"): 1115.6e6 + 58.0e6,
-                  (NACA_WORKLOAD, "k_lusgs_sweep"): 42.97e6 + 0.04e6}
+KERNEL_TRAFFIC = {(WORKLOAD, "k_lusgs_sweep"): 397.4e6 + 62.2e6,
+                  (NACA_WORKLOAD, "k_lusgs_sweep"): 11.04e6}
 # The whole iteration's compulsory footprint (FP64): read q, dxidx, inv_j,
 # write q, dq* write+read = 30 words per node; SA adds nut r/w, dist, the
 # alpha/beta/gamma tensors and dnut* w/r = 44 words.
