@@ -1335,7 +1335,10 @@ int do_iteration_crank() {
 // computed on the second stream beside the LU-SGS sweeps, into g.d_out, and
 // g.ev_resid marks its end.
 // With retirement on: every block whose status word is non-zero stops (its
-// live flag drops to 0 for the whole step).
+// live flag drops to 0 for the whole step).  It runs before every step, in the
+// first step of a call before the primitives that open it: a field that is
+// already bad when the call begins is marked by those primitives, takes that
+// step, and is dropped by the next one.
 int do_retire() {
   if (!g.retire) return AERO_OK;
   const int nb = (int)g.blocks.size();
@@ -1349,17 +1352,17 @@ int do_retire() {
 // the start of the next one, so the steps of one call compute them once per
 // iteration, at its end (where a block that has failed is marked before the
 // next step's k_retire), and before the first (opening_primitives): one pass
-// over the boxes less per step, 25 of the plate's 1350 us.
+// over the boxes less per step, 25 of the plate's 1350 us.  Every further step
+// of a call follows a do_retire of its own.
 int opening_primitives() {
   int rc;
-  if (crank_on()) return AERO_OK;  // (each of its sub-iterations computes them)
   if ((rc = do_retire())) return rc;
+  if (crank_on()) return AERO_OK;  // (each of its sub-iterations computes them)
   return do_getpri_all();
 }
 
 int do_iteration(bool want_dt_minmax, bool resid_beside = false) {
   int rc;
-  if ((rc = do_retire())) return rc;
   if (crank_on()) return do_iteration_crank();
   int nb = (int)g.blocks.size();
   // inviscid_flux_1 (rhsi and its face scratch) beside viscous_flux and
@@ -1801,7 +1804,7 @@ int aero_autotune(int iters) {
     if ((r = step_once())) return r;  // warm
     CK(cudaEventRecord(a, g.stream));
     for (int x = 0; x < iters; ++x)
-      if ((r = step_once())) return r;
+      if ((r = do_retire()) || (r = step_once())) return r;
     CK(cudaEventRecord(b, g.stream));
     CK(cudaEventSynchronize(b));
     float f = 0.f;
@@ -3027,6 +3030,7 @@ int aero_step(int nsteps, double* resid_hist, double* dt_minmax) {
   for (int s0 = 0; s0 < nsteps; s0 += kHistSteps) {
     const int n = std::min(kHistSteps, nsteps - s0);
     for (int s = s0; s < s0 + n; ++s) {
+      if (s > 0 && (rc = do_retire())) return rc;
       if (s == nsteps - 1 && dt_minmax != nullptr) {
         if ((rc = do_iteration(true))) return rc;
         if ((rc = do_getpri_all())) return rc;  // end of the time step (main.f90:434-447)
