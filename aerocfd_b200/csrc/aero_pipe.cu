@@ -166,8 +166,8 @@ __global__ void k_pipe_index(const BlockView* __restrict__ blocks) {
     wh |= (unsigned)fh << (10 * e);
   }
   const double word = __longlong_as_double((long long)((unsigned long long)(wh | flags) << 32 | (wl | flags)));
-  P.rec[(long)kPipeRec * pos + PW_NBR] = word;
-  P.sa_rec[(long)kPipeSaRec * pos + SW_NBR] = word;
+  if (P.rec) P.rec[(long)kPipeRec * pos + PW_NBR] = word;  // (a view holds the records of its own sweeps only)
+  if (P.sa_rec) P.sa_rec[(long)kPipeSaRec * pos + SW_NBR] = word;
 }
 
 #ifdef __CUDACC__  // (the order's tables above also build as host code, for their test)

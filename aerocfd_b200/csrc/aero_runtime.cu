@@ -14,6 +14,7 @@
 #include <cstring>
 #include <map>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "../../include/aerocfd_gpu.h"
@@ -22,6 +23,10 @@
 #include "aero_topology.h"
 
 using namespace aero;
+
+extern "C" {
+static void release_case();
+}
 
 namespace {
 
@@ -37,6 +42,7 @@ struct HostBlock {
   long plane = 0;
   size_t arena_off = 0;  // doubles
   void* ws = nullptr;    // LU-SGS workspace (one allocation)
+  size_t ws_bytes = 0;
   bool own_params = false;  // aero_set_block_params: this block's case constants
   double params[7] = {};
   CaseConsts cc{};
@@ -154,6 +160,15 @@ constexpr long kPollBudgetMax = 1L << 20;
 // Steps whose residuals aero_step keeps on their way to the host at a time.
 constexpr int kHistSteps = 256;
 
+// Which sweeps a view's workspace serves: the pipelined ones or the ones that
+// aero_set_sweep_cluster / aero_set_sa_sweep_cluster select, or neither.
+struct WsNeed {
+  bool pipe = false, other = false;        // mean flow
+  bool sa_pipe = false, sa_other = false;  // SA equation
+  bool any_pipe() const { return pipe || sa_pipe; }
+  bool any_other() const { return other || sa_other; }
+};
+
 struct State {
   bool inited = false;
   int device = 0;
@@ -193,6 +208,7 @@ struct State {
   // CTAs), the one of a drop-in call's own view, and per precision the dynamic
   // shared memory set so far and whether clusters of 16 are allowed
   PipeFit pipe, tpipe, pipe_sa, tpipe_sa;
+  WsNeed ws_need;  // what the registered blocks' workspaces are laid out for
   size_t smem_pipe_sa = 0;
   size_t smem_pipe[2][kPipeVariants] = {};
   bool np_pipe[2][kPipeVariants] = {};
@@ -439,11 +455,8 @@ size_t view_doubles(long plane) {
   return s;
 }
 void fill_view(BlockView& v, const Box& b, const Box& b0, const Box& b1, long plane, double* base) {
+  v = BlockView{};
   v.b = b; v.b0 = b0; v.b1 = b1;
-  v.ccb = nullptr;
-  v.pipe = PipeView{};
-  v.bstat = nullptr;
-  v.live = nullptr;
   v.nx = b.nx(); v.ny = b.ny();
   v.plane = plane;
   size_t off = 0;
@@ -453,20 +466,43 @@ void fill_view(BlockView& v, const Box& b, const Box& b0, const Box& b1, long pl
   }
 }
 
-// LU-SGS workspace of one view (see BlockView): one device allocation holding
-// poff, rec_f, rec_b, sca, dqs, dq, sa_rec, sa_dq, nat, nbr, pidx, seg and the
-// pipelined sweeps' arrays, each array starting on a 256-byte boundary (the sweeps' bulk copies and L2 prefetches
-// of plane chunks need 16-byte aligned starts).
+// LU-SGS workspace of one view (see BlockView): one device allocation with the
+// arrays of the sweeps in `need` (poff, rec_f, rec_b, sca, dqs, dq, sa_rec,
+// sa_dq, nat, nbr, pidx and seg of the other sweeps, the pipelined sweeps'
+// records and order), each starting on a 256-byte boundary (the sweeps' bulk
+// copies and L2 prefetches of plane chunks need 16-byte aligned starts).  The
+// pipelined sweeps take 452 bytes per updated node, the others 1540, so a view
+// holds what its sweeps use and no more.  lay_out points v's arrays into ws
+// and returns the bytes (ws null: the bytes only).
 constexpr size_t kWsAlign = 256;
-constexpr int kWsArrays = 17;
 long pipe_plane_max(const Box& b1) { return (long)kPipeSlabs * (b1.nx() + b1.ny() + b1.nz()); }
-size_t ws_round(size_t bytes) { return (bytes + kWsAlign - 1) / kWsAlign * kWsAlign; }
-size_t workspace_bytes(const Box& b1, int H) {
-  size_t N1 = (size_t)b1.size();
-  return (size_t)(H + 1) * sizeof(long) + N1 * (2 * kRec + kSca + 8 + 5 + kSaRec + 1) * sizeof(double) +
-         N1 * sizeof(long) + N1 * 7 * sizeof(int) + (size_t)H * (b1.nz() + 2) * sizeof(int) +
-         N1 * ((kPipeRec + kPipeSaRec) * sizeof(double) + sizeof(int)) +
-         (size_t)pipe_plane_max(b1) * sizeof(PipePlane) + (kPipeSlabs + 1) * sizeof(int) + (kWsArrays + 1) * kWsAlign;
+size_t lay_out(BlockView& v, void* ws, const WsNeed& need) {
+  const size_t N1 = (size_t)v.b1.size(), H = (size_t)std::max(0, v.b1.nx() + v.b1.ny() + v.b1.nz() - 2);
+  size_t off = 0;
+  auto take = [&](auto*& p, bool on, size_t n) {
+    p = nullptr;
+    if (!on) return;
+    if (ws) p = reinterpret_cast<std::remove_reference_t<decltype(p)>>((char*)ws + off);
+    off += (n * sizeof(*p) + kWsAlign - 1) / kWsAlign * kWsAlign;
+  };
+  take(v.rec_f, need.other, N1 * kRec);
+  take(v.rec_b, need.other, N1 * kRec);
+  take(v.sca, need.other, N1 * kSca);
+  take(v.dqs, need.other, N1 * 8);
+  take(v.dq, need.other, N1 * 5);
+  take(v.sa_rec, need.sa_other, N1 * kSaRec);
+  take(v.sa_dq, need.sa_other, N1);
+  take(v.nat, need.any_other(), N1);
+  take(v.poff, need.any_other(), H + 1);
+  take(v.nbr, need.any_other(), N1 * 7);
+  v.pidx = v.nbr ? v.nbr + 6 * N1 : nullptr;
+  take(v.seg, need.any_other(), H * (v.b1.nz() + 2));
+  take(v.pipe.rec, need.pipe, N1 * kPipeRec);
+  take(v.pipe.sa_rec, need.sa_pipe, N1 * kPipeSaRec);
+  take(v.pipe.at, need.any_pipe(), N1);
+  take(v.pipe.plane, need.any_pipe(), (size_t)pipe_plane_max(v.b1));
+  take(v.pipe.slab, need.any_pipe(), kPipeSlabs + 1);
+  return off + kWsAlign;
 }
 // The order of a view's pipelined sweeps for clusters of ncta CTAs: its tables
 // into the view's workspace (k_pipe_index then fills the per-node ones).
@@ -479,38 +515,21 @@ int set_pipe_order(BlockView& v, int ncta) {
                      g.stream));
   return AERO_OK;
 }
-int attach_workspace(BlockView& v, void* ws, const std::vector<long>& poff, int pmax) {
-  size_t N1 = (size_t)v.b1.size();
-  char* p = (char*)ws;
-  auto take = [&](size_t bytes) {
-    char* at = p;
-    p += ws_round(bytes);
-    return at;
-  };
+// lay_out, with the tables of `need` that come from the host: the plane
+// offsets and segments, the pipelined sweeps' order for clusters of C CTAs.
+int attach_workspace(BlockView& v, void* ws, const WsNeed& need, int C) {
+  int pmax = 0;
+  const std::vector<long> poff = plane_offsets(v.b1, pmax);
   v.nplanes = (int)poff.size() - 1;
   v.pmax = pmax;
-  v.rec_f = (double*)take(N1 * kRec * sizeof(double));
-  v.rec_b = (double*)take(N1 * kRec * sizeof(double));
-  v.sca = (double*)take(N1 * kSca * sizeof(double));
-  v.dqs = (double*)take(N1 * 8 * sizeof(double));
-  v.dq = (double*)take(N1 * 5 * sizeof(double));
-  v.sa_rec = (double*)take(N1 * kSaRec * sizeof(double));
-  v.sa_dq = (double*)take(N1 * sizeof(double));
-  v.nat = (long*)take(N1 * sizeof(long));
-  v.poff = (long*)take(poff.size() * sizeof(long));
-  v.nbr = (int*)take(N1 * 7 * sizeof(int));
-  v.pidx = v.nbr + 6 * N1;
-  const std::vector<int> seg = plane_segments(v.b1);
-  v.seg = (int*)take(seg.size() * sizeof(int));
-  v.pipe.rec = (double*)take(N1 * kPipeRec * sizeof(double));
-  v.pipe.sa_rec = (double*)take(N1 * kPipeSaRec * sizeof(double));
-  v.pipe.at = (int*)take(N1 * sizeof(int));
-  v.pipe.plane = (PipePlane*)take((size_t)pipe_plane_max(v.b1) * sizeof(PipePlane));
-  v.pipe.slab = (int*)take((kPipeSlabs + 1) * sizeof(int));
-  CK(cudaMemcpyAsync(v.poff, poff.data(), poff.size() * sizeof(long), cudaMemcpyHostToDevice, g.stream));
-  if (!seg.empty())
-    CK(cudaMemcpyAsync(v.seg, seg.data(), seg.size() * sizeof(int), cudaMemcpyHostToDevice, g.stream));
-  return AERO_OK;
+  lay_out(v, ws, need);
+  if (need.any_other()) {
+    const std::vector<int> seg = plane_segments(v.b1);
+    CK(cudaMemcpyAsync(v.poff, poff.data(), poff.size() * sizeof(long), cudaMemcpyHostToDevice, g.stream));
+    if (!seg.empty())
+      CK(cudaMemcpyAsync(v.seg, seg.data(), seg.size() * sizeof(int), cudaMemcpyHostToDevice, g.stream));
+  }
+  return need.any_pipe() ? set_pipe_order(v, C) : AERO_OK;
 }
 
 // The kernel of the pipelined sweeps, ready for launches of this shape.
@@ -740,19 +759,6 @@ int resolve(const Box& b, const Box& b0, const Box& b1, const std::vector<Arg>& 
   if (!g.d_tview) CK(cudaMalloc(&g.d_tview, sizeof(BlockView)));
   CK(cudaMemsetAsync(g.t_arena, 0, need * sizeof(double), g.stream));
   fill_view(t.view, b, b0, b1, plane, g.t_arena);
-  if (b1.nx() > 0 && b1.ny() > 0 && b1.nz() > 0) {
-    int pmax = 0;
-    std::vector<long> poff = plane_offsets(b1, pmax);
-    size_t wsb = workspace_bytes(b1, (int)poff.size() - 1);
-    if (wsb > g.t_ws_bytes) {
-      if (g.t_ws) CK(cudaFree(g.t_ws));
-      g.t_ws = nullptr;
-      CK(cudaMalloc(&g.t_ws, wsb));
-      g.t_ws_bytes = wsb;
-    }
-    int rc2 = attach_workspace(t.view, g.t_ws, poff, pmax);
-    if (rc2) return rc2;
-  }
   CK(cudaMemcpyAsync(g.d_tview, &t.view, sizeof(BlockView), cudaMemcpyHostToDevice, g.stream));
   t.d_view = g.d_tview;
   t.resident = false;
@@ -1097,14 +1103,16 @@ int launch_implicit(const BlockView* views, int nblk, long maxExt, long maxN1, i
   return AERO_OK;
 }
 
-int launch_pipe_index(const BlockView* views, int nblk, long maxN1) {
-  PROF(P_INDEX, (k_pipe_index<<<dim3(cdiv(maxN1, 256), nblk), 256, 0, g.stream>>>(views)));
-  CKL();
-  return AERO_OK;
-}
-int launch_index(const BlockView* views, int nblk, long maxN1) {
-  PROF(P_INDEX, (k_plane_index<<<dim3(cdiv(maxN1, 256), nblk), 256, 0, g.stream>>>(views)));
-  CKL();
+// The per-node index tables of the sweeps that the views' workspaces serve.
+int launch_index(const BlockView* views, int nblk, long maxN1, const WsNeed& need) {
+  if (need.any_pipe()) {
+    PROF(P_INDEX, (k_pipe_index<<<dim3(cdiv(maxN1, 256), nblk), 256, 0, g.stream>>>(views)));
+    CKL();
+  }
+  if (need.any_other()) {
+    PROF(P_INDEX, (k_plane_index<<<dim3(cdiv(maxN1, 256), nblk), 256, 0, g.stream>>>(views)));
+    CKL();
+  }
   return AERO_OK;
 }
 
@@ -1173,36 +1181,95 @@ int upload_views() {
   return AERO_OK;
 }
 
+// What the selected sweeps of the registered blocks need.
+WsNeed needed() {
+  const bool p = g.tune.pipe && g.pipe.ok, sp = g.tune.sa_pipe && g.pipe_sa.ok;
+  return WsNeed{p, !p, sp, !sp};
+}
+
+// The registered blocks' workspaces laid out for `need` and the order of
+// g.pipe.C, the views on the device and their index tables.
+int lay_out_blocks(const WsNeed& need) {
+  const int nb = (int)g.blocks.size();
+  CK(cudaStreamSynchronize(g.stream));
+  for (int m = 0; m < nb; ++m) {
+    HostBlock& H = g.blocks[m];
+    const size_t bytes = lay_out(g.views[m], nullptr, need);
+    if (bytes > H.ws_bytes) {
+      CK(cudaFree(H.ws));
+      H.ws = nullptr;
+      H.ws_bytes = 0;
+      CK(cudaMalloc(&H.ws, bytes));
+      H.ws_bytes = bytes;
+    }
+    int rc = attach_workspace(g.views[m], H.ws, need, g.pipe.C);
+    if (rc) return rc;
+  }
+  int rc = upload_views();
+  if (rc) return rc;
+  g.ws_need = need;
+  return launch_index(g.d_blocks, nb, g.max_b1, need);
+}
+
+// After a change of the selected sweeps or (reorder) of the pipelined ones'
+// order: the workspaces they need.  A device without room for them takes the
+// change back (undo), keeps the workspaces it had and reports AERO_ERR_NOMEM.
+template <class F>
+int relayout(bool reorder, F undo) {
+  graph_release();
+  if (!g.setup) return AERO_OK;
+  const WsNeed need = needed();
+  if (!reorder && need.pipe == g.ws_need.pipe && need.sa_pipe == g.ws_need.sa_pipe) return AERO_OK;
+  const int rc = lay_out_blocks(need);
+  if (rc == AERO_OK) return rc;
+  cudaGetLastError();
+  const std::string why = g.err;
+  undo();
+  if (lay_out_blocks(needed()) != AERO_OK) release_case();  // no room for what fitted before: the case is gone
+  g.err = why;
+  return rc;
+}
+
 // The registered blocks' pipelined sweeps on clusters of C CTAs (1, 2, 4, 8
-// or 16): the order's tables again, and the views that hold them.  *fits is
-// false (and nothing changes) when a plane or such a cluster does not fit.
+// or 16).  *fits is false (and nothing changes) when a plane or such a cluster
+// does not fit.
 int set_pipe_cluster(int C, bool* fits) {
   const int nb = (int)g.blocks.size();
   const PipeFit f = pipe_fit(g.views.data(), nb, C);
   *fits = f.ok;
   if (!f.ok) return AERO_OK;
+  const PipeFit pipe = g.pipe, pipe_sa = g.pipe_sa;
   g.pipe = f;
   g.pipe_sa = pipe_sa_fit(g.views.data(), nb, C);
-  for (int m = 0; m < nb; ++m) {
-    int rc = set_pipe_order(g.views[m], C);
-    if (rc) return rc;
-  }
-  int rc = upload_views();
-  if (rc) return rc;
-  graph_release();
-  return launch_pipe_index(g.d_blocks, nb, g.max_b1);
+  return relayout(true, [&] {
+    g.pipe = pipe;
+    g.pipe_sa = pipe_sa;
+  });
 }
 
-// The sweeps' orders of a drop-in call's own view.
-int transient_order(BlockTarget& t, long N1) {
+// The workspace and the sweeps' orders of a drop-in call's own view: those of
+// the mean flow (sa false) or of the SA equation.
+int transient_order(BlockTarget& t, bool sa) {
+  const Box& b1 = t.view.b1;
+  if (b1.nx() < 1 || b1.ny() < 1 || b1.nz() < 1) return fail(AERO_ERR_ARG, "the updated index box is empty");
   g.tpipe = pipe_choose(&t.view, 1);
-  g.tpipe_sa = pipe_sa_fit(&t.view, 1, g.tpipe.C);
-  int rc = set_pipe_order(t.view, g.tpipe.C);
+  if (sa) g.tpipe_sa = pipe_sa_fit(&t.view, 1, g.tpipe.C);
+  WsNeed need;
+  if (sa)
+    (g.tune.sa_pipe && g.tpipe_sa.ok ? need.sa_pipe : need.sa_other) = true;
+  else
+    (g.tune.pipe && g.tpipe.ok ? need.pipe : need.other) = true;
+  const size_t bytes = lay_out(t.view, nullptr, need);
+  if (bytes > g.t_ws_bytes) {
+    if (g.t_ws) CK(cudaFree(g.t_ws));
+    g.t_ws = nullptr;
+    CK(cudaMalloc(&g.t_ws, bytes));
+    g.t_ws_bytes = bytes;
+  }
+  int rc = attach_workspace(t.view, g.t_ws, need, g.tpipe.C);
   if (rc) return rc;
   CK(cudaMemcpyAsync(g.d_tview, &t.view, sizeof(BlockView), cudaMemcpyHostToDevice, g.stream));
-  if ((rc = launch_pipe_index(t.d_view, 1, N1))) return rc;
-  const bool all = g.tune.pipe && g.tpipe.ok && g.tune.sa_pipe && g.tpipe_sa.ok;
-  return all ? AERO_OK : launch_index(t.d_view, 1, N1);
+  return launch_index(t.d_view, 1, b1.size(), need);
 }
 
 bool viscous_on() { return g.cc.solver == IFLAG_NSSOLVER; }
@@ -1560,6 +1627,7 @@ static void release_case() {
       if (H.pinned[f]) cudaHostUnregister(H.host[f]);
     if (H.ws) cudaFree(H.ws);
     H.ws = nullptr;
+    H.ws_bytes = 0;
   }
   g.blocks.clear();
   g.registry.clear();
@@ -1929,9 +1997,10 @@ int aero_set_sweep_cluster(int ctas) {
   if (ctas == 16 && !bulk_cluster16_fits() && !slab_cluster16_fits(5))
     return fail(AERO_ERR_ARG, "a cluster of 16 sweep CTAs does not fit this device or these blocks "
                               "(16 CTAs take the bulk or the slab exchange only)");
+  const State::Tune was = g.tune;
   g.tune.sweep_cl = ctas == 1 ? 0 : ctas;
   g.tune.pipe = false;
-  graph_release();
+  if ((rc = relayout(false, [&] { g.tune = was; }))) return rc;
   set_tuning_text();
   return AERO_OK;
 }
@@ -1963,9 +2032,10 @@ int aero_set_sa_sweep_cluster(int ctas) {
     return fail(AERO_ERR_ARG, "SA sweep cluster of %d CTAs is not 1, 2, 4, 8 or 16", ctas);
   if (ctas == 16 && !slab_cluster16_fits(1))
     return fail(AERO_ERR_ARG, "a cluster of 16 SA sweep CTAs does not fit this device or these blocks");
+  const State::Tune was = g.tune;
   g.tune.sa_cl = ctas == 1 ? 0 : ctas;
   g.tune.sa_pipe = false;
-  graph_release();
+  if ((rc = relayout(false, [&] { g.tune = was; }))) return rc;
   set_tuning_text();
   return AERO_OK;
 }
@@ -2170,16 +2240,11 @@ int aero_finish_setup(void) {
     HostBlock& H = g.blocks[m];
     fill_view(g.views[m], H.b, H.b0, H.b1, H.plane, g.arena + H.arena_off);
     int pmax = 0;
-    std::vector<long> poff = plane_offsets(H.b1, pmax);
-    CK(cudaMalloc(&H.ws, workspace_bytes(H.b1, (int)poff.size() - 1)));
-    if ((rc = attach_workspace(g.views[m], H.ws, poff, pmax))) return rc;
+    g.hmax_all = std::max(g.hmax_all, (int)plane_offsets(H.b1, pmax).size() - 1);
     g.pmax_all = std::max(g.pmax_all, pmax);
-    g.hmax_all = std::max(g.hmax_all, (int)poff.size() - 1);
   }
   g.pipe = pipe_choose(g.views.data(), nb);
   g.pipe_sa = pipe_sa_fit(g.views.data(), nb, g.pipe.C);
-  for (int m = 0; m < nb; ++m)
-    if ((rc = set_pipe_order(g.views[m], g.pipe.C))) return rc;
   // per-block case constants of a batch (aero_set_block_params)
   bool any_own = false;
   for (auto& H : g.blocks) any_own = any_own || H.own_params;
@@ -2207,7 +2272,7 @@ int aero_finish_setup(void) {
   CK(cudaMalloc(&g.d_init, nb * sizeof(InitValues)));
   CK(cudaMalloc(&g.d_blocks, nb * sizeof(BlockView)));
   CK(cudaMalloc(&g.d_blocks_chain, nb * sizeof(BlockView)));
-  if ((rc = upload_views())) return rc;
+  if ((rc = lay_out_blocks(needed()))) return rc;
   // tables
   CK(cudaMalloc(&g.d_bc_ops, std::max<size_t>(1, topo.bc_ops.size()) * sizeof(BcOp)));
   if (!topo.bc_ops.empty())
@@ -2249,9 +2314,6 @@ int aero_finish_setup(void) {
   if (g.nhalo) CK(cudaMemcpyAsync(g.d_halo, topo.halo.data(), g.nhalo * sizeof(HaloEntry), cudaMemcpyHostToDevice, g.stream));
   if (g.navg_src) CK(cudaMemcpyAsync(g.d_avg_src, topo.avg_src.data(), g.navg_src * sizeof(AvgSrc), cudaMemcpyHostToDevice, g.stream));
   if (g.navg_dst) CK(cudaMemcpyAsync(g.d_avg_dst, topo.avg_dst.data(), g.navg_dst * sizeof(AvgDst), cudaMemcpyHostToDevice, g.stream));
-  if ((rc = launch_index(g.d_blocks, nb, g.max_b1))) return rc;
-  if ((rc = launch_pipe_index(g.d_blocks, nb, g.max_b1))) return rc;
-  if ((rc = launch_pipe_index(g.d_blocks, nb, g.max_b1))) return rc;
   g.resid_ctas = (int)cdiv(g.max_b1, 256);
   CK(cudaMalloc(&g.d_part, (size_t)g.resid_ctas * nb * 6 * sizeof(double)));
   CK(cudaMalloc(&g.d_resid_blocks, (size_t)nb * 7 * sizeof(double)));
@@ -2608,7 +2670,7 @@ int aero_implicit1st(double* q, const double* dt, const double* pri_v, double* r
   CaseConsts cc = consts_with(*gamma, g.cc.cv, g.cc.re);
   cc.cfl = *cfl;
   Box e = grown_box(b, b1);
-  if (!t.resident && (rc = transient_order(t, b1.size()))) return rc;
+  if (!t.resident && (rc = transient_order(t, false))) return rc;
   if ((rc = launch_implicit(t.d_view, 1, e.size(), b1.size(), t.view.pmax, t.view.nplanes, cc,
                             t.resident ? g.pipe : g.tpipe, nullptr, true, nullptr, &t.view)))
     return rc;
@@ -2820,7 +2882,7 @@ int aero_sa_model(double* nut, double* sa_rhs, const double* dt, const double* p
   if ((rc = resolve(b, b0, b1, args, t))) return rc;
   CaseConsts cc = consts_with(g.cc.gamma, g.cc.cv, *re);
   cc.cfl = *cfl;
-  if (!t.resident && (rc = transient_order(t, b1.size()))) return rc;
+  if (!t.resident && (rc = transient_order(t, true))) return rc;
   if ((rc = launch_sa(t.d_view, 1, b.size(), b1.size(), t.view.pmax, cc, t.resident ? g.pipe_sa : g.tpipe_sa, nullptr,
                       &t.view)))
     return rc;
