@@ -127,6 +127,14 @@ struct PipeSmem {
     words = planes + H;
   }
 };
+// Messages between the posts of a sweep's counts of messages read, and the most
+// groups that these allow.  The groups post after their planes, in no order
+// among themselves, so the count in place may be the one of a group that is
+// NG - 1 planes, (NG - 1) / lot posts, behind; a sender of message m needs a
+// count above m - D once all before m have been read, the last lot - 1 of them
+// unposted: lot + (NG - 1) / lot * lot < D.
+__host__ __device__ constexpr int pipe_lot(int D) { return D < 4 ? 1 : D / 4; }
+__host__ __device__ constexpr int pipe_groups(int D) { return 3 * pipe_lot(D); }
 // a poll budget of this many polls means the time bound of the cluster waits
 constexpr long kPipePolls = 1L << 20;
 __global__ void k_pipe_index(const BlockView* __restrict__ blocks);

@@ -572,7 +572,7 @@ __device__ __forceinline__ void pipe_body(const BlockView* __restrict__ blocks, 
     const int TG2 = 2 * 32 * W;
     const unsigned read_lo = cut.has_lo ? slab::map(slab::local(&s_read[1]), me - 1) : 0u;
     const unsigned read_hi = cut.has_hi ? slab::map(slab::local(&s_read[0]), me + 1) : 0u;
-    const int lot = max(1, D / 4);
+    const int lot = pipe_lot(D);
     const unsigned sm_at = slab::local(sm), step_b8 = 8u * (unsigned)step_b;
     // Once a stage's wait has run out the warp reads no stage any more (a later
     // phase of a stage whose copies never came would pass for complete) and
@@ -761,7 +761,7 @@ __device__ __forceinline__ void pipe_body(const BlockView* __restrict__ blocks, 
             const int m = cut.out(FWD, h, me);
             const int* count = &s_read[FWD ? 1 : 0];
             // (the groups post their counts in no particular order, so a count may
-            // be followed by a smaller one: what counts is to have seen it)
+            // be followed by a smaller one; pipe_groups keeps that one large enough)
             bool room = m < D || slab::load_relaxed(count) > m - D;
             if (!room) wait_bounded([&] { return (room = slab::load_relaxed(count) > m - D) || s_abort != 0; });
             if (room) {

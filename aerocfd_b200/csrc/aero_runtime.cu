@@ -546,46 +546,23 @@ int prepare_pipe(const PipeFit& pf, int f) {
   return AERO_OK;
 }
 
+PipeNeed pipe_need(const BlockView* hv, int nblk, int C) {
+  PipeNeed n;
+  for (int m = 0; m < nblk; ++m) n.add(hv[m].b1, C);
+  return n;
+}
+
 PipeFit pipe_fit(const BlockView* hv, int nblk, int C) {
   PipeFit f;
   f.C = C;
-  int P = 1, L = 1, H = 1, steps = 1, cuts = 1;
-  for (int m = 0; m < nblk; ++m) {
-    const PipeTables t = pipe_tables(hv[m].b1, pipe_direction(hv[m].b1, C), C);
-    P = std::max(P, t.pmax);
-    L = std::max(L, t.lmax);
-    H = std::max(H, t.hmax);
-    steps = std::max(steps, 2 * (hv[m].b1.nx() + hv[m].b1.ny() + hv[m].b1.nz() - 2));
-    cuts = std::max(cuts, t.ce);
-  }
-  if (P > 1022) return f;  // the neighbour words' index range
-  PipeShape& s = f.sh;
-  s.P = P;
-  s.L = L;
-  auto bytes = [&] { return (size_t)PipeSmem(s, kPipeRec, kPipeProd, 5, H).words * sizeof(double); };
-  // one CTA of up to 16 warps per SM or, where the clusters outnumber the SMs
-  // and two stages of a plane fit half of one, two of up to 8
-  bool two = nblk * C > kSms;
-  size_t limit = 0;
-  for (;; two = false) {
-    limit = (size_t)(two ? 113 : 226) * 1024;
-    s.W = std::min(two ? 7 : 15, (P + 9) / 10);  // compute warps
-    // up to seven groups while the CTA keeps to 8 warps (200 registers each),
-    // else two within 11 (168 registers)
-    s.NG = s.W <= 3 ? 7 / s.W : (!two && s.W <= 5) ? 2 : 1;
-    s.NST = s.NG + 3;
-    s.D = 8;
-    while (bytes() > limit && s.NST > std::max(2, s.NG)) --s.NST;
-    while (bytes() > limit && s.NG > 1) s.NST = std::max(2, --s.NG);
-    if (bytes() <= limit) break;
-    if (!two) return f;
-  }
-  // more messages on the way while three quarters of that hold them
-  while (s.D < 64 && (s.D *= 2, bytes() <= limit / 4 * 3)) {
-  }
-  if (s.D > 8 && bytes() > limit / 4 * 3) s.D /= 2;
-  f.smem = bytes();
-  f.threads = 32 * (s.W * s.NG + 1);
+  const PipeNeed need = pipe_need(hv, nblk, C);
+  const PipeLaunch pl = pipe_launch(need, nblk * C, kSms);
+  if (!pl.ok) return f;
+  f.sh = pl.sh;
+  f.smem = pl.smem;
+  f.threads = pl.threads;
+  const bool two = pl.two;
+  const PipeShape& s = f.sh;
   f.variant = two ? 3 : 0;
   while (kPipeWarps[f.variant] < s.W * s.NG + 1) ++f.variant;
   // the clusters of this shape that the device holds at a time
@@ -619,40 +596,19 @@ PipeFit pipe_fit(const BlockView* hv, int nblk, int C) {
   // behind a cut starts about 600 after the one before it.
   const double step = two ? 1400.0 + 130.0 * s.W
                           : std::max(560.0, (1700.0 + (s.W > 10 ? 240.0 : 150.0) * s.W) / s.NG);
-  const int passes = (P + 10 * s.W - 1) / (10 * s.W);
-  f.est = ((nblk + active - 1) / active) * (steps * step * passes + 1200.0 * cuts);
+  const int passes = (s.P + 10 * s.W - 1) / (10 * s.W);
+  f.est = ((nblk + active - 1) / active) * (need.steps * step * passes + 1200.0 * need.cuts);
   return f;
 }
 
 PipeFit pipe_sa_fit(const BlockView* hv, int nblk, int C) {
   PipeFit f;
   f.C = C;
-  int P = 1, L = 1, H = 1;
-  for (int m = 0; m < nblk; ++m) {
-    const PipeTables t = pipe_tables(hv[m].b1, pipe_direction(hv[m].b1, C), C);
-    P = std::max(P, t.pmax);
-    L = std::max(L, t.lmax);
-    H = std::max(H, t.hmax);
-  }
-  if (P > 1022) return f;
-  PipeShape& s = f.sh;
-  s.P = P;
-  s.L = L;
-  // a node's step is short (a division and a barrier), so its records are read
-  // up to four planes ahead; at most a quarter of the SM's shared memory, which
-  // the mean flow's CTAs beside it need
-  s.W = std::min(15, (P + 31) / 32);
-  s.NG = std::max(1, std::min(4, 15 / s.W));
-  s.NST = s.NG + 3;
-  s.D = 8;
-  auto bytes = [&] { return (size_t)PipeSmem(s, kPipeSaRec, 1, 1, H).words * sizeof(double); };
-  while (bytes() > 56 * 1024 && s.NST > std::max(2, s.NG)) --s.NST;
-  if (bytes() > 200 * 1024) return f;
-  while (s.D < 64 && (s.D *= 2, bytes() <= 56 * 1024)) {
-  }
-  if (s.D > 8 && bytes() > 56 * 1024) s.D /= 2;
-  f.smem = bytes();
-  f.threads = 32 * (s.W * s.NG + 1);
+  const PipeLaunch pl = pipe_sa_launch(pipe_need(hv, nblk, C));
+  if (!pl.ok) return f;
+  f.sh = pl.sh;
+  f.smem = pl.smem;
+  f.threads = pl.threads;
   if (f.smem > g.smem_pipe_sa) {
     if (cudaFuncSetAttribute(k_pipe_sa_sweep, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)f.smem) != cudaSuccess ||
         cudaFuncSetAttribute(k_pipe_sa_sweep, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {

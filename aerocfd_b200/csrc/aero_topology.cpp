@@ -391,4 +391,74 @@ int pipe_direction(const Box& b1, int ncta) {
   return best;
 }
 
+void PipeNeed::add(const Box& b1, int ncta) {
+  const PipeTables t = pipe_tables(b1, pipe_direction(b1, ncta), ncta);
+  P = std::max(P, t.pmax);
+  L = std::max(L, t.lmax);
+  H = std::max(H, t.hmax);
+  steps = std::max(steps, 2 * (b1.nx() + b1.ny() + b1.nz() - 2));
+  cuts = std::max(cuts, t.ce);
+}
+
+PipeLaunch pipe_launch(const PipeNeed& need, long ctas, int sms) {
+  PipeLaunch f;
+  if (need.P > 1022) return f;  // the neighbour words' index range
+  PipeShape& s = f.sh;
+  s.P = need.P;
+  s.L = need.L;
+  auto bytes = [&] { return (size_t)PipeSmem(s, kPipeRec, kPipeProd, 5, need.H).words * sizeof(double); };
+  // one CTA of up to 16 warps per SM or, where the clusters outnumber the SMs
+  // and two stages of a plane fit half of one, two of up to 8
+  f.two = ctas > sms;
+  size_t limit = 0;
+  for (;; f.two = false) {
+    limit = (size_t)(f.two ? 113 : 226) * 1024;
+    s.W = std::min(f.two ? 7 : 15, (s.P + 9) / 10);  // compute warps
+    // up to seven groups while the CTA keeps to 8 warps (200 registers each),
+    // else two within 11 (168 registers)
+    s.NG = s.W <= 3 ? 7 / s.W : (!f.two && s.W <= 5) ? 2 : 1;
+    s.NST = s.NG + 3;
+    s.D = 8;
+    while (bytes() > limit && s.NST > std::max(2, s.NG)) --s.NST;
+    while (bytes() > limit && s.NG > 1) s.NST = std::max(2, --s.NG);
+    if (bytes() <= limit) break;
+    if (!f.two) return f;
+  }
+  // more messages on the way while three quarters of that hold them
+  while (s.D < 64 && (s.D *= 2, bytes() <= limit / 4 * 3)) {
+  }
+  if (s.D > 8 && bytes() > limit / 4 * 3) s.D /= 2;
+  s.NG = std::min(s.NG, pipe_groups(s.D));  // (7 to 6 where a slab's plane table leaves room for 8 messages only)
+  f.smem = bytes();
+  f.threads = 32 * (s.W * s.NG + 1);
+  f.ok = true;
+  return f;
+}
+
+PipeLaunch pipe_sa_launch(const PipeNeed& need) {
+  PipeLaunch f;
+  if (need.P > 1022) return f;
+  PipeShape& s = f.sh;
+  s.P = need.P;
+  s.L = need.L;
+  // a node's step is short (a division and a barrier), so its records are read
+  // up to four planes ahead; at most a quarter of the SM's shared memory, which
+  // the mean flow's CTAs beside it need
+  s.W = std::min(15, (s.P + 31) / 32);
+  s.NG = std::max(1, std::min(4, 15 / s.W));
+  s.NST = s.NG + 3;
+  s.D = 8;
+  auto bytes = [&] { return (size_t)PipeSmem(s, kPipeSaRec, 1, 1, need.H).words * sizeof(double); };
+  while (bytes() > 56 * 1024 && s.NST > std::max(2, s.NG)) --s.NST;
+  if (bytes() > 200 * 1024) return f;
+  while (s.D < 64 && (s.D *= 2, bytes() <= 56 * 1024)) {
+  }
+  if (s.D > 8 && bytes() > 56 * 1024) s.D /= 2;
+  s.NG = std::min(s.NG, pipe_groups(s.D));
+  f.smem = bytes();
+  f.threads = 32 * (s.W * s.NG + 1);
+  f.ok = true;
+  return f;
+}
+
 }  // namespace aero

@@ -60,4 +60,24 @@ constexpr int kPipeSlabs = 16;
 // long one leaves few and wide ones).
 int pipe_direction(const Box& b1, int ncta);
 
+// What a set of blocks asks of the pipelined sweeps on clusters of one size:
+// the largest plane P, message L and slab H (planes), the most plane steps of
+// both passes and the most slabs of a block.
+struct PipeNeed {
+  int P = 1, L = 1, H = 1, steps = 1, cuts = 1;
+  void add(const Box& b1, int ncta);
+};
+// Their launch shape, ok false where a plane does not fit: threads and dynamic
+// shared memory of a CTA; two: two CTAs per SM.
+struct PipeLaunch {
+  bool ok = false, two = false;
+  PipeShape sh{};
+  int threads = 0;
+  size_t smem = 0;
+};
+// The mean flow's, for `ctas` CTAs in all on a device of `sms` SMs, and the SA
+// equation's.
+PipeLaunch pipe_launch(const PipeNeed& need, long ctas, int sms);
+PipeLaunch pipe_sa_launch(const PipeNeed& need);
+
 }  // namespace aero
