@@ -110,7 +110,6 @@ __global__ void __launch_bounds__(256) k_crank_lines(const BlockView* __restrict
   const int line0 = blockIdx.x * lpc;
   if (line0 >= lines) return;
   const int nl = min(lpc, lines - line0);
-  const long st = d == 0 ? 1 : (d == 1 ? (long)B.nx : (long)B.nx * B.ny);
   const int cb = 3 * d + 1;
   const double inv1 = 1.0 + kAlph;
   // word w of node x (-1 .. len) of line l; the row stride is odd, so threads on

@@ -30,9 +30,6 @@ static void release_case();
 
 namespace {
 
-// Streaming multiprocessors of the device the launch shapes are made for.
-constexpr int kSms = 148;
-
 struct HostBlock {
   bool used = false;
   Box b{}, b0{}, b1{};
@@ -172,6 +169,7 @@ struct WsNeed {
 struct State {
   bool inited = false;
   int device = 0;
+  int sms = 1;  // streaming multiprocessors of the device (148 on a whole B200)
   cudaStream_t stream = nullptr;
   // second stream of a steady iteration: inviscid_flux_1 runs on it beside
   // viscous_flux and find_dt, and sa_model beside implicit1st (in each pair
@@ -556,7 +554,7 @@ PipeFit pipe_fit(const BlockView* hv, int nblk, int C) {
   PipeFit f;
   f.C = C;
   const PipeNeed need = pipe_need(hv, nblk, C);
-  const PipeLaunch pl = pipe_launch(need, nblk * C, kSms);
+  const PipeLaunch pl = pipe_launch(need, (long)nblk * C, g.sms);
   if (!pl.ok) return f;
   f.sh = pl.sh;
   f.smem = pl.smem;
@@ -1296,7 +1294,7 @@ int launch_crank(const BlockView* views, int nblk, long maxN, long maxN1, const 
   int lpc[3] = {4, 4, 4};
   for (int d = 0; d < dirs; ++d) {
     fit = fit && crank_lines_smem(len[d], 4) <= kSmem;
-    lpc[d] = (int)std::min<long>(32, std::max<long>(4, cdiv(nl[d] * nblk, kSms)));
+    lpc[d] = (int)std::min<long>(32, std::max<long>(4, cdiv(nl[d] * nblk, g.sms)));
     while (lpc[d] > 4 && crank_lines_smem(len[d], lpc[d]) > kSmem) --lpc[d];
   }
   if (fit) {
@@ -1535,6 +1533,7 @@ const char* aero_last_error(void) { return g.err.c_str(); }
 int aero_init(int device) {
   if (g.inited) return AERO_OK;
   CK(cudaSetDevice(device));
+  CK(cudaDeviceGetAttribute(&g.sms, cudaDevAttrMultiProcessorCount, device));
   g.smem_pipe_sa = 0;
   for (int f = 0; f < 2; ++f) {
     g.smem_staged[f] = 0;

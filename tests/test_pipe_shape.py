@@ -85,3 +85,12 @@ def test_launch_shapes(tmp_path):
     subprocess.run(["g++", "-x", "c++", "-std=c++17", "-O2", "-w", "-I" + csrc, str(src), "-o", str(exe)], check=True)
     out = subprocess.run([str(exe)], capture_output=True, text=True)
     assert out.returncode == 0, out.stdout
+
+
+def test_the_device_gives_the_number_of_sms():
+    """No launch shape is made for a number of SMs written into the source."""
+    import re
+    csrc = os.path.join(ROOT, "aerocfd_b200", "csrc")
+    for name in ("aero_runtime.cu", "aero_topology.cpp", "aero_topology.h", "aero_kernels.h"):
+        code = re.sub(r"//[^\n]*", "", open(os.path.join(csrc, name)).read())
+        assert not re.search(r"\b148\b", code), name
