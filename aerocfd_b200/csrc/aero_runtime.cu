@@ -1960,6 +1960,45 @@ int aero_set_sweep_cluster(int ctas) {
   return AERO_OK;
 }
 
+int aero_set_sweep_pipeline(int ctas) {
+  int rc = need_init();
+  if (rc) return rc;
+  if (ctas != 0 && ctas != 1 && ctas != 2 && ctas != 4 && ctas != 8 && ctas != 16)
+    return fail(AERO_ERR_ARG, "pipelined sweeps on %d CTAs: not 0 (by rule), 1, 2, 4, 8 or 16", ctas);
+  if (ctas && (rc = need_setup())) return rc;
+  const int nb = (int)g.blocks.size();
+  const PipeFit pipe = g.pipe, pipe_sa = g.pipe_sa;
+  if (g.setup) {
+    const PipeFit f = ctas ? pipe_fit(g.views.data(), nb, ctas) : pipe_choose(g.views.data(), nb);
+    if (ctas && !f.ok)
+      return fail(AERO_ERR_ARG, "the pipelined sweeps of these blocks do not fit clusters of %d CTAs on this device", ctas);
+    g.pipe = f;
+    g.pipe_sa = pipe_sa_fit(g.views.data(), nb, f.C);
+  }
+  const State::Tune was = g.tune;
+  g.tune.pipe = g.tune.sa_pipe = true;
+  if (!ctas) g.tune.sweep_cl = g.tune.sa_cl = 0;
+  if ((rc = relayout(true, [&] {
+         g.tune = was;
+         g.pipe = pipe;
+         g.pipe_sa = pipe_sa;
+       })))
+    return rc;
+  set_tuning_text();
+  return AERO_OK;
+}
+
+int aero_get_sweep_pipeline(int* out8) {
+  int rc = need_setup();
+  if (rc) return rc;
+  const PipeFit& f = g.pipe;
+  const PipeShape& s = f.sh;
+  const int v[8] = {f.C, kPipeCtas[f.variant], s.W, s.NG, s.NST, s.D, s.P, 0};
+  for (int x = 0; x < 8; ++x) out8[x] = g.tune.pipe && f.ok ? v[x] : 0;
+  out8[7] = g.tune.sa_pipe && g.pipe_sa.ok ? g.pipe_sa.C : 0;
+  return AERO_OK;
+}
+
 int aero_set_sweep_prefetch(int planes) {
   int rc = need_init();
   if (rc) return rc;

@@ -134,8 +134,22 @@ class GpuCase:
         _lib.check(self.L.aero_set_tuning(ctypes.c_int(inv_tile), ctypes.c_int(ew), ctypes.c_int(visc),
                                           ctypes.c_int(mats), ctypes.c_int(nst_max)), "aero_set_tuning")
 
+    def set_sweep_pipeline(self, ctas: int = 0) -> None:
+        """aero_set_sweep_pipeline: the pipelined sweeps (the default) on
+        clusters of 1, 2, 4, 8 or 16 CTAs per block, or (0) as the rule gives."""
+        _lib.check(self.L.aero_set_sweep_pipeline(ctypes.c_int(ctas)), "aero_set_sweep_pipeline")
+
+    def sweep_pipeline(self) -> dict:
+        """aero_get_sweep_pipeline: the pipelined sweeps' shape in use (ctas 0:
+        other sweeps run)."""
+        out = np.zeros(8, dtype=np.int32)
+        _lib.check(self.L.aero_get_sweep_pipeline(_p_int(out)), "aero_get_sweep_pipeline")
+        names = ("ctas", "per_sm", "warps", "groups", "stages", "messages", "plane", "sa_ctas")
+        return dict(zip(names, out.tolist()))
+
     def set_sweep_cluster(self, ctas: int) -> None:
-        """aero_set_sweep_cluster: CTAs per block of the LU-SGS sweep (1, 2, 4, 8, 16)."""
+        """aero_set_sweep_cluster: CTAs per block of the LU-SGS sweep (1, 2, 4,
+        8, 16) in place of the pipelined one."""
         _lib.check(self.L.aero_set_sweep_cluster(ctypes.c_int(ctas)), "aero_set_sweep_cluster")
 
     def set_sweep_exchange(self, mode) -> None:
@@ -158,7 +172,7 @@ class GpuCase:
 
     def set_sa_sweep_cluster(self, ctas: int) -> None:
         """aero_set_sa_sweep_cluster: CTAs per block of the SA sweep (1, 2, 4,
-        8, 16), pipelined by k-slabs."""
+        8, 16), by k-slabs, in place of the pipelined one."""
         _lib.check(self.L.aero_set_sa_sweep_cluster(ctypes.c_int(ctas)), "aero_set_sa_sweep_cluster")
 
     def set_poll_budget(self, polls: int) -> None:

@@ -98,7 +98,18 @@ module aerocfd_gpu
       integer(c_int) :: zones(*)
     end function
 
-    ! CTAs per block of the LU-SGS sweep: 1, 2, 4 or 8 (no counterpart in the reference)
+    ! the pipelined LU-SGS sweeps (the default): CTAs per block 0 (by rule), 1,
+    ! 2, 4, 8 or 16, and the shape in use (no counterpart in the reference)
+    integer(c_int) function aero_set_sweep_pipeline(ctas) bind(C, name="aero_set_sweep_pipeline")
+      import :: c_int
+      integer(c_int), value :: ctas
+    end function
+    integer(c_int) function aero_get_sweep_pipeline(out8) bind(C, name="aero_get_sweep_pipeline")
+      import :: c_int
+      integer(c_int) :: out8(8)
+    end function
+
+    ! other LU-SGS sweeps: CTAs per block 1, 2, 4, 8 or 16 (no counterpart in the reference)
     integer(c_int) function aero_set_sweep_cluster(ctas) bind(C, name="aero_set_sweep_cluster")
       import :: c_int
       integer(c_int), value :: ctas

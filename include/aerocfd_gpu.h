@@ -350,9 +350,21 @@ const char* aero_tuning(void);
  * the mixed face kernel bounded for 10), 32, 64 or 128; element-wise threads 128, 256,
  * 512; viscous and block-record threads 64, 128, 256; sweep stages 2..4. */
 int aero_set_tuning(int inv_tile, int ew, int visc, int mats, int nst_max);
-/* By default each block's LU-SGS sweeps run as a pipeline of slabs over a
- * cluster whose size a rule or the autotuner chooses, where the planes fit.
- * This call selects another sweep instead, by the CTAs that share a block: 1
+/* By default each block's LU-SGS sweeps, the mean flow's and the SA equation's,
+ * run as a pipeline of slabs over a cluster of CTAs, where the planes fit.  This
+ * call selects them again after aero_set_sweep_cluster or
+ * aero_set_sa_sweep_cluster: ctas = 0 with the cluster size that the rule of
+ * aero_finish_setup gives (and, for blocks that do not fit, the sweeps of one
+ * CTA per block, as after set-up); ctas = 1, 2, 4, 8 or 16 with that size
+ * (after aero_finish_setup; AERO_ERR_ARG, and nothing changes, when the planes
+ * or such clusters do not fit).  The arithmetic is the same for every choice. */
+int aero_set_sweep_pipeline(int ctas);
+/* The pipelined sweeps in use: out8 = CTAs per block, CTAs per SM, warps of a
+ * group, groups, stages, inbox messages and the largest plane (nodes) of the
+ * mean flow's, all 0 when other sweeps run; then the CTAs per block of the SA
+ * equation's (0: other sweeps). */
+int aero_get_sweep_pipeline(int* out8);
+/* This call selects another sweep instead, by the CTAs that share a block: 1
  * (one CTA per block, the records staged in shared memory when its planes fit) or a thread-block
  * cluster of 2, 4 or 8 CTAs, or 16 CTAs (a non-portable cluster size, with
  * the bulk-copy or the slab exchange only; accepted after aero_finish_setup
