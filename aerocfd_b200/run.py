@@ -37,12 +37,12 @@ def main(argv=None) -> int:
     ap.add_argument("--warmup", type=int, default=3)
     ap.add_argument("--inviscid", type=int, default=4, help="4 Roe + WENO3, 5 SW + WENO5, 8 WCNS5")
     ap.add_argument("--mixed", action="store_true")
-    ap.add_argument("--sweep-cluster", type=int, default=0, help="CTAs per block of the LU-SGS sweep (0: autotune)")
+    ap.add_argument("--sweep-cluster", type=int, default=0, help="CTAs per block of the LU-SGS sweep in place of the pipelined one (0: autotune)")
     ap.add_argument("--sweep-exchange", choices=["l2", "shared", "slab", "shared2"], default=None,
-                    help="plane exchange of a cluster sweep (default: the autotuner's or L2)")
-    ap.add_argument("--sa-sweep-cluster", type=int, default=0, help="CTAs per block of the SA sweep (0: autotune)")
+                    help="plane exchange of a cluster sweep (of 8 CTAs unless --sweep-cluster says; default: L2)")
+    ap.add_argument("--sa-sweep-cluster", type=int, default=0, help="CTAs per block of the SA sweep in place of the pipelined one (0: autotune)")
     ap.add_argument("--sweep-prefetch", type=int, choices=[2, 3, 4], default=0,
-                    help="L2 prefetch distance of the bulk-exchange sweep (default: the autotuner's)")
+                    help="L2 prefetch distance of the bulk-exchange sweep (--sweep-exchange shared; default: the autotuner's)")
     ap.add_argument("--register-bound", type=int, choices=[0, 1], default=None,
                     help="register-bounded viscous part a (default: the autotuner's)")
     ap.add_argument("--no-graphs", action="store_true")
@@ -62,8 +62,8 @@ def main(argv=None) -> int:
             tuning = ""
         else:
             tuning = "" if args.no_autotune else gc.autotune(3)
-        if args.sweep_cluster:
-            gc.set_sweep_cluster(args.sweep_cluster)
+        if args.sweep_cluster or args.sweep_exchange:  # (the pipelined sweeps have no exchange to choose)
+            gc.set_sweep_cluster(args.sweep_cluster or 8)
         if args.sweep_exchange:
             gc.set_sweep_exchange(args.sweep_exchange)
         if args.sa_sweep_cluster:

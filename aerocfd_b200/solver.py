@@ -153,7 +153,8 @@ class GpuCase:
         _lib.check(self.L.aero_set_sweep_cluster(ctypes.c_int(ctas)), "aero_set_sweep_cluster")
 
     def set_sweep_exchange(self, mode) -> None:
-        """aero_set_sweep_exchange: how a cluster shares a sweep: "l2" (or
+        """aero_set_sweep_exchange: how a cluster that set_sweep_cluster
+        selected shares a sweep: "l2" (or
         False), "shared" (or True: bulk copies between shared memories),
         "slab" (CTAs pipelined by k-slabs) or "shared2" (bulk copies, two CTAs
         per SM)."""

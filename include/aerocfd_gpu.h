@@ -371,7 +371,9 @@ int aero_get_sweep_pipeline(int* out8);
  * when the device can hold such a cluster).  The arithmetic is the same for
  * every choice. */
 int aero_set_sweep_cluster(int ctas);
-/* How a cluster's CTAs share a block's sweep: 0 (default) every CTA a part
+/* How the CTAs of the clusters that aero_set_sweep_cluster selects share a
+ * block's sweep (the pipelined sweeps have no such choice: the setting waits
+ * until clusters are selected): 0 (default) every CTA a part
  * of each hyperplane, the values passed through L2 with a cluster barrier
  * per plane; 1 the same with bulk copies between the CTAs' shared memories
  * counted on mbarriers (used when every row of the largest plane has its own
@@ -393,8 +395,8 @@ int aero_set_sa_sweep_cluster(int ctas);
  * is the same either way; aero_autotune chooses it too. */
 int aero_set_register_bound(int on);
 /* Planes ahead (2, the default, 3 or 4) at which the bulk-exchange sweep's
- * CTAs prefetch their shares of the plane records into L2.  Results are the
- * same for every choice; aero_autotune chooses it too. */
+ * CTAs (aero_set_sweep_cluster with exchange 1 or 3) prefetch their shares of
+ * the plane records into L2.  Results are the same for every choice; aero_autotune chooses it too. */
 int aero_set_sweep_prefetch(int planes);
 /* Polls each bounded wait of the staged LU-SGS sweep (one CTA per block)
  * makes before it gives up, 0..1048576 (the default); each poll may suspend
