@@ -418,14 +418,34 @@ int fail(int code, const char* fmt, ...) {
   return code;
 }
 
+// (A reported error is cleared, so that the next call's check of its launches
+// does not report it once more.)
 #define CK(call)                                                                          \
   do {                                                                                    \
     cudaError_t e_ = (call);                                                              \
-    if (e_ != cudaSuccess)                                                                \
+    if (e_ != cudaSuccess) {                                                              \
+      cudaGetLastError();                                                                 \
       return fail(e_ == cudaErrorMemoryAllocation ? AERO_ERR_NOMEM : AERO_ERR_CUDA,       \
                   "%s failed: %s (%s:%d)", #call, cudaGetErrorString(e_), __FILE__, __LINE__); \
+    }                                                                                     \
   } while (0)
 #define CKL() CK(cudaGetLastError())
+
+// At least n elements at p, which holds `have` of them (its contents are lost
+// when it grows; after a failed allocation it holds none).
+template <class T>
+int grow(T*& p, size_t& have, size_t n) {
+  if (n <= have) return AERO_OK;
+  cudaFree(p);
+  p = nullptr;
+  have = 0;
+  if constexpr (std::is_void_v<T>)
+    CK(cudaMalloc(&p, n));
+  else
+    CK(cudaMalloc(&p, n * sizeof(T)));
+  have = n;
+  return AERO_OK;
+}
 
 long round32(long n) { return (n + 31) / 32 * 32; }
 unsigned cdiv(long a, long b) { return (unsigned)((a + b - 1) / b); }
@@ -629,14 +649,7 @@ PipeFit pipe_choose(const BlockView* hv, int nblk) {
   return best;
 }
 
-int ensure_staging(size_t doubles) {
-  if (doubles <= g.staging_doubles) return AERO_OK;
-  if (g.d_staging) CK(cudaFree(g.d_staging));
-  g.d_staging = nullptr;
-  CK(cudaMalloc(&g.d_staging, doubles * sizeof(double)));
-  g.staging_doubles = doubles;
-  return AERO_OK;
-}
+int ensure_staging(size_t doubles) { return grow(g.d_staging, g.staging_doubles, doubles); }
 
 // host (c, i, j, k) column-major <-> one field of a view
 int upload(const double* host, double* dev_field, long n, int nc, long plane) {
@@ -704,12 +717,8 @@ int resolve(const Box& b, const Box& b0, const Box& b1, const std::vector<Arg>& 
     return fail(AERO_ERR_ARG, "index box with %d k-planes in a %d-D configuration", b.nz(), dim);
   long plane = round32(b.size());
   size_t need = view_doubles(plane);
-  if (need > g.t_doubles) {
-    if (g.t_arena) CK(cudaFree(g.t_arena));
-    g.t_arena = nullptr;
-    CK(cudaMalloc(&g.t_arena, need * sizeof(double)));
-    g.t_doubles = need;
-  }
+  int rc = grow(g.t_arena, g.t_doubles, need);
+  if (rc) return rc;
   if (!g.d_tview) CK(cudaMalloc(&g.d_tview, sizeof(BlockView)));
   CK(cudaMemsetAsync(g.t_arena, 0, need * sizeof(double), g.stream));
   fill_view(t.view, b, b0, b1, plane, g.t_arena);
@@ -718,7 +727,7 @@ int resolve(const Box& b, const Box& b0, const Box& b1, const std::vector<Arg>& 
   t.resident = false;
   t.m = -1;
   for (const Arg& a : args) {
-    int rc = upload(a.host, t.view.f[a.fid], b.size(), field_nc(a.fid), plane);
+    rc = upload(a.host, t.view.f[a.fid], b.size(), field_nc(a.fid), plane);
     if (rc) return rc;
   }
   return AERO_OK;
@@ -1148,16 +1157,8 @@ int lay_out_blocks(const WsNeed& need) {
   CK(cudaStreamSynchronize(g.stream));
   for (int m = 0; m < nb; ++m) {
     HostBlock& H = g.blocks[m];
-    const size_t bytes = lay_out(g.views[m], nullptr, need);
-    if (bytes > H.ws_bytes) {
-      CK(cudaFree(H.ws));
-      H.ws = nullptr;
-      H.ws_bytes = 0;
-      CK(cudaMalloc(&H.ws, bytes));
-      H.ws_bytes = bytes;
-    }
-    int rc = attach_workspace(g.views[m], H.ws, need, g.pipe.C);
-    if (rc) return rc;
+    int rc = grow(H.ws, H.ws_bytes, lay_out(g.views[m], nullptr, need));
+    if (rc || (rc = attach_workspace(g.views[m], H.ws, need, g.pipe.C))) return rc;
   }
   int rc = upload_views();
   if (rc) return rc;
@@ -1176,7 +1177,6 @@ int relayout(bool reorder, F undo) {
   if (!reorder && need.pipe == g.ws_need.pipe && need.sa_pipe == g.ws_need.sa_pipe) return AERO_OK;
   const int rc = lay_out_blocks(need);
   if (rc == AERO_OK) return rc;
-  cudaGetLastError();
   const std::string why = g.err;
   undo();
   if (lay_out_blocks(needed()) != AERO_OK) release_case();  // no room for what fitted before: the case is gone
@@ -1213,15 +1213,8 @@ int transient_order(BlockTarget& t, bool sa) {
     (g.tune.sa_pipe && g.tpipe_sa.ok ? need.sa_pipe : need.sa_other) = true;
   else
     (g.tune.pipe && g.tpipe.ok ? need.pipe : need.other) = true;
-  const size_t bytes = lay_out(t.view, nullptr, need);
-  if (bytes > g.t_ws_bytes) {
-    if (g.t_ws) CK(cudaFree(g.t_ws));
-    g.t_ws = nullptr;
-    CK(cudaMalloc(&g.t_ws, bytes));
-    g.t_ws_bytes = bytes;
-  }
-  int rc = attach_workspace(t.view, g.t_ws, need, g.tpipe.C);
-  if (rc) return rc;
+  int rc = grow(g.t_ws, g.t_ws_bytes, lay_out(t.view, nullptr, need));
+  if (rc || (rc = attach_workspace(t.view, g.t_ws, need, g.tpipe.C))) return rc;
   CK(cudaMemcpyAsync(g.d_tview, &t.view, sizeof(BlockView), cudaMemcpyHostToDevice, g.stream));
   return launch_index(t.d_view, 1, b1.size(), need);
 }
