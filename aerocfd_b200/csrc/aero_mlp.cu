@@ -23,6 +23,7 @@ namespace {
   do {                                                                                 \
     cudaError_t e_ = (call);                                                           \
     if (e_ != cudaSuccess) {                                                           \
+      cudaGetLastError(); /* reported here, not by the next call's check */            \
       char b_[200];                                                                    \
       std::snprintf(b_, sizeof b_, "%s: %s", #call, cudaGetErrorString(e_));           \
       return set_last_error(e_ == cudaErrorMemoryAllocation ? AERO_ERR_NOMEM : AERO_ERR_CUDA, b_); \
@@ -395,38 +396,53 @@ struct Net {
   unsigned* status = nullptr;
   long n_all = 0;
   int adam_t = 0;
-  std::vector<void*> allocs;
-  char* arena = nullptr;  // rest of the newest allocation
-  size_t arena_left = 0;
+  char* arena = nullptr;  // the arrays above but xall, tall and perm
+  size_t arena_bytes = 0;
 } g_net;
 
 constexpr int kSplitMax = 32;
 
-// The network's arrays share a few device allocations (each of at least
-// kArenaBytes); an array starts on a 256-byte boundary.
-constexpr size_t kArenaBytes = (size_t)256 << 20;
+// Elements of the largest layer's side.
+size_t widest() { return (size_t)std::max(g_net.width, 128); }
+
+// The next n elements of the network's one device allocation, from a 256-byte
+// boundary on (null while the bytes are only counted).
 template <class T>
-int alloc(T*& p, size_t n) {
-  p = nullptr;
-  const size_t bytes = (n * sizeof(T) + 255) / 256 * 256;
-  if (bytes > g_net.arena_left) {
-    void* a = nullptr;
-    const size_t size = std::max(bytes, kArenaBytes);
-    if (cudaMalloc(&a, size) != cudaSuccess)
-      return set_last_error(AERO_ERR_NOMEM, "warm-start network: device allocation failed");
-    g_net.allocs.push_back(a);
-    cudaMemset(a, 0, size);
-    g_net.arena = (char*)a;
-    g_net.arena_left = size;
+void take(T*& p, size_t n) {
+  p = g_net.arena ? (T*)(g_net.arena + g_net.arena_bytes) : nullptr;
+  g_net.arena_bytes += (n * sizeof(T) + 255) / 256 * 256;
+}
+int loss_parts() { return g_net.nout / 32 * (g_net.batch / kTileRows); }
+void lay_out() {
+  Net& N = g_net;
+  const size_t B = N.batch, W = widest();
+  N.arena_bytes = 0;
+  for (Layer& y : N.L) {
+    const size_t nw = (size_t)y.nin * y.nout, nb = y.nout;
+    take(y.w, nw); take(y.b, nb); take(y.mw, nw); take(y.vw, nw); take(y.mb, nb);
+    take(y.vb, nb); take(y.gw, nw); take(y.gb, nb); take(y.wb, nw); take(y.wt, nw);
   }
-  p = (T*)g_net.arena;
-  g_net.arena += bytes;
-  g_net.arena_left -= bytes;
-  return AERO_OK;
+  for (int l = 0; l <= N.depth; ++l) {
+    const size_t n = B * (l == 0 ? N.kin : N.width);
+    take(N.h[l], n);
+    take(N.ht[l], n);
+  }
+  for (int l = 0; l < N.depth; ++l) take(N.z[l], B * N.width);
+  take(N.c_out, B * N.nout);
+  take(N.y, B * N.n_out);
+  take(N.dh, B * N.width);
+  take(N.d, B * W);
+  take(N.dt, B * W);
+  take(N.scratch, kSplitMax * W * W);
+  take(N.cpart, B / kTileRows * W);
+  take(N.lpart, (size_t)loss_parts());
+  take(N.xb, B * N.n_in);
+  take(N.tb, B * N.n_out);
+  take(N.status, (size_t)1);
 }
 
 void release() {
-  for (void* p : g_net.allocs) cudaFree(p);
+  cudaFree(g_net.arena);
   cudaFree(g_net.xall);
   cudaFree(g_net.tall);
   cudaFree(g_net.perm[0]);
@@ -465,8 +481,6 @@ int forward(const float* x, const int* idx, int n, bool with_back) {
   }
   return gemm_parts(N.h[N.depth], N.L[N.depth].wb, N.c_out, B, N.nout, N.width, one, N.status, 0);
 }
-
-int loss_parts() { return g_net.nout / 32 * (g_net.batch / kTileRows); }
 
 // Backward pass of the last forward with the targets t (rows as forward's): the
 // loss parts and, layer by layer, the gradients into gw, gb or (train) an Adam
@@ -540,16 +554,26 @@ int aero_mlp_create(int n_in, int n_out, int width, int depth, int batch, unsign
   Net& N = g_net;
   N.n_in = n_in; N.n_out = n_out; N.width = width; N.depth = depth; N.batch = batch;
   int rc;
+  N.L.resize(depth + 1);
+  N.h.resize(depth + 1);
+  N.ht.resize(depth + 1);
+  N.z.resize(depth);
+  for (int l = 0; l <= depth; ++l) {
+    N.L[l].nin = l == 0 ? N.kin : width;
+    N.L[l].nout = l == depth ? N.nout : width;
+  }
+  lay_out();
+  if (cudaMalloc(&N.arena, N.arena_bytes) != cudaSuccess) {
+    cudaGetLastError();
+    release();
+    return set_last_error(AERO_ERR_NOMEM, "warm-start network: device allocation failed");
+  }
+  MCK(cudaMemset(N.arena, 0, N.arena_bytes));
+  lay_out();
   uint64_t s = seed;
   for (int l = 0; l <= depth; ++l) {
-    Layer y;
-    y.nin = l == 0 ? N.kin : width;
-    y.nout = l == depth ? N.nout : width;
-    size_t nw = (size_t)y.nin * y.nout;
-    if ((rc = alloc(y.w, nw)) || (rc = alloc(y.b, y.nout)) || (rc = alloc(y.mw, nw)) || (rc = alloc(y.vw, nw)) ||
-        (rc = alloc(y.mb, y.nout)) || (rc = alloc(y.vb, y.nout)) || (rc = alloc(y.gw, nw)) ||
-        (rc = alloc(y.gb, y.nout)) || (rc = alloc(y.wb, nw)) || (rc = alloc(y.wt, nw)))
-      return rc;
+    const Layer& y = N.L[l];
+    const size_t nw = (size_t)y.nin * y.nout;
     // Glorot-uniform over the real fan-in / fan-out; padded rows/columns stay 0
     int fin = l == 0 ? n_in : width, fout = l == depth ? n_out : width;
     double a = std::sqrt(6.0 / (fin + fout));
@@ -568,25 +592,7 @@ int aero_mlp_create(int n_in, int n_out, int width, int depth, int batch, unsign
     }
     MCK(cudaMemcpy(y.w, w.data(), nw * 4, cudaMemcpyHostToDevice));
     MCK(cudaMemcpy(y.wb, wb.data(), nw * 2, cudaMemcpyHostToDevice));
-    N.L.push_back(y);
   }
-  N.h.resize(depth + 1);
-  N.ht.resize(depth + 1);
-  N.z.resize(depth);
-  for (int l = 0; l <= depth; ++l) {
-    const size_t n = (size_t)batch * (l == 0 ? N.kin : width);
-    if ((rc = alloc(N.h[l], n)) || (rc = alloc(N.ht[l], n))) return rc;
-  }
-  for (int l = 0; l < depth; ++l)
-    if ((rc = alloc(N.z[l], (size_t)batch * width))) return rc;
-  size_t wmax = (size_t)std::max(width, 128);
-  if ((rc = alloc(N.c_out, (size_t)batch * N.nout)) || (rc = alloc(N.y, (size_t)batch * n_out)) ||
-      (rc = alloc(N.dh, (size_t)batch * width)) || (rc = alloc(N.d, (size_t)batch * wmax)) ||
-      (rc = alloc(N.dt, (size_t)batch * wmax)) || (rc = alloc(N.scratch, (size_t)kSplitMax * wmax * wmax)) ||
-      (rc = alloc(N.cpart, (size_t)(batch / kTileRows) * wmax)) || (rc = alloc(N.lpart, (size_t)loss_parts())) ||
-      (rc = alloc(N.xb, (size_t)batch * n_in)) || (rc = alloc(N.tb, (size_t)batch * n_out)) ||
-      (rc = alloc(N.status, 1)))
-    return rc;
   for (auto k : {(const void*)k_activate, (const void*)k_back_hidden, (const void*)k_back_output})
     MCK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTileSmem));
   if ((rc = refresh_transposes())) return rc;

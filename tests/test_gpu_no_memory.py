@@ -48,6 +48,21 @@ def test_a_box_that_no_device_holds(gpu):
     L.aero_finalize()
 
 
+def test_a_network_that_no_device_holds(gpu):
+    """32 layers of 1024 on 20 million rows (5 TB) are refused; the next network
+    trains."""
+    from aerocfd_b200 import warmstart
+    L = _lib.load()
+    assert L.aero_mlp_create(5, 4, 1024, 32, 512 * 40000, ctypes.c_ulonglong(1)) == ERR_NOMEM
+    net = warmstart.Network(n_in=5, n_out=4, width=128, depth=2, batch=512)
+    try:
+        rng = np.random.default_rng(0)
+        loss = net.train(rng.uniform(-1, 1, (1024, 5)), rng.uniform(-1, 1, (1024, 4)), 4)
+        assert np.all(np.isfinite(loss)) and np.all(loss > 0)
+    finally:
+        net.close()
+
+
 def test_sweeps_whose_workspace_does_not_fit(gpu):
     """aero_set_sweep_cluster on a full device keeps the sweeps that run, and
     the run goes on to the same bits; with room it is accepted."""
