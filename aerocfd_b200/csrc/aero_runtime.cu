@@ -1836,13 +1836,14 @@ int aero_autotune(int iters) {
   const bool piped = g.tune.pipe && g.pipe.ok;
   struct Knob { int* v; std::vector<int> cand; };
   std::vector<Knob> knobs = {{&g.tune.inv_tile, {0, -6, -8, -10, 32, 64, 128}}, {&g.tune.ew, {128, 256, 512}},
-                             {&g.tune.visc, {64, 128, 256}}, {&g.tune.mats, {64, 128, 256}},
-                             {&g.tune.bound, {0, 1}}};
+                             {&g.tune.visc, {64, 128, 256}}, {&g.tune.bound, {0, 1}}};
+  // (the block-record threads, stages, exchange and prefetch distance are the other sweeps')
   if (piped) {
     knobs.push_back({&pipe_c, {}});
     for (int C : {1, 2, 4, 8, 16})
       if (pipe_fit(g.views.data(), nb, C).ok) knobs.back().cand.push_back(C);
   } else {
+    knobs.push_back({&g.tune.mats, {64, 128, 256}});
     knobs.push_back({&g.tune.nst_max, {2, 3, 4}});
     knobs.push_back({&sweep_mode, {0, 8, 16, 32, 9, 17, 33, 10, 18, 34, 11, 19, 35}});
     if (bulk_cluster16_fits()) knobs.back().cand.push_back(65);   // 16 CTAs, bulk exchange
