@@ -24,7 +24,9 @@ restatement of the reference's algorithm (the reference is Fortran + MPI and
 cannot be compiled in this image) on the host cores, one thread per block
 like one MPI rank per block.
 
-Extra objects on the line: `mixed` (the device-timed metric with
+The last line of stdout is the one JSON line, the headline metric and what
+qualifies it; a line `details: {...}` before it repeats that and adds the extra
+objects: `tuning`, `kernels`, `iteration_roofline`, `mixed` (the device-timed metric with
 aero_set_precision(1), and the mixed solution's max / L2 error against FP64
 after 50 iterations from one state), `naca` (the laminar NACA0012 O-grid
 4 x 129 x 65 x 3, M 0.5, Re 5000, AoA 2, CFL 2: the same measurements, its own
@@ -864,6 +866,19 @@ def measure(solver, case, workload: str, args, world: int, local: int, dist, clo
     return out
 
 
+# Keys of the one JSON line; the objects under them keep the keys named here.
+HEADLINE = ("metric", "value", "unit", "n_gpus", "steps", "warmup", "ms_per_step", "higher_is_better", "scaling",
+            "vs_baseline", "dtype", "data", "config", "clocks", "e2e", "gpu_launches", "device_status", "roofline")
+HEADLINE_PARTS = {"roofline": ("bound", "kernel", "achieved", "unit", "frac", "ms_per_launch")}
+
+
+def headline(line: dict) -> dict:
+    """What the last line of stdout holds of a full result: short enough
+    (about 1.3 kB) to stay whole where only the end of the output is kept."""
+    return {k: {p: line[k][p] for p in HEADLINE_PARTS[k]} if k in HEADLINE_PARTS else line[k]
+            for k in HEADLINE if k in line}
+
+
 def main():
     args = parse()
     rank = int(os.environ.get("RANK", "0"))
@@ -899,8 +914,7 @@ def main():
     if m["device_status"]:
         print(f"warning: device status word {m['device_status']}", file=sys.stderr)
     config.update({"l2": "flushed (256 MiB write) before every timed step; the case's arrays exceed L2",
-                   "execution": "each step replayed from a CUDA graph; launch shapes from the autotuner: "
-                                + m.pop("tuning"),
+                   "execution": "each step replayed from a CUDA graph; launch shapes from the autotuner",
                    "parallelism": f"replicas x{world}"})
     line = {"metric": "Mcell-iter/s", "value": m.pop("value"), "unit": "Mcell-iter/s", "n_gpus": world,
             "steps": args.steps, "warmup": args.warmup, "ms_per_step": m.pop("ms_per_step"),
@@ -953,7 +967,8 @@ def main():
                         "reference's layout for a 1-block case"}
         line["convergence"] = conv
     if rank == 0:
-        print(json.dumps(line))
+        print("details: " + json.dumps(line))
+        print(json.dumps(headline(line)))
     if dist:
         dist.barrier()
         dist.destroy_process_group()
