@@ -18,8 +18,13 @@
 // With the blocks read from memory instead, one plane step moved 76 words per
 // node through shared memory twice and through HBM once, which bounded it.
 // What bounds it now is the FP64 rate, about 780 operations per node and pass,
-// or, for small planes, the chain from plane to plane (two divisions, two
-// products and a barrier, about 350 cycles).
+// or, for small planes, the step from plane to plane.  Its chain of dependent
+// operations (two divisions, two products, a barrier) adds up to about 340
+// cycles; measured are 576 a step for aerofoil blocks of 129 x 65 x 3 on 8 CTAs
+// (112 us over 382 steps at 1965 MHz, the start behind the cuts included), 670 for a
+// channel of 97 x 49 x 5 on 16 and 870 for one of 33 x 17 x 5 on 8 (both with about 8
+// us of launch): the rest is the other groups' block formation, which shares
+// the chain's FP64 pipe, and the hand-over between the groups.
 //
 // The arithmetic per node is the reference's, operation by operation (calc_jm,
 // the products summed column by column, the three directions added in their

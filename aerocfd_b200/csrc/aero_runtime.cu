@@ -150,8 +150,9 @@ PipeFit pipe_sa_fit(const BlockView* hv, int nblk, int C);
 // nblk host views hv.
 SlabFit slab_fit_for(const BlockView* hv, int nblk, int ncta, int rows);
 
-// Largest (and default) number of polls of each wait of the staged LU-SGS
-// sweep, the kernel's own bound.
+// Largest (and default) number of polls of each wait for staged records (the
+// pipelined mean-flow sweep, which takes the default as its time bound, and the
+// one-CTA staged sweep, whose own bound it is).
 constexpr long kPollBudgetMax = 1L << 20;
 
 // Steps whose residuals aero_step keeps on their way to the host at a time.
@@ -210,7 +211,7 @@ struct State {
   size_t smem_pipe_sa = 0;
   size_t smem_pipe[2][kPipeVariants] = {};
   bool np_pipe[2][kPipeVariants] = {};
-  long spin_limit = kPollBudgetMax;  // polls of each staged-sweep wait (aero_set_poll_budget)
+  long spin_limit = kPollBudgetMax;  // polls of each wait for staged records (aero_set_poll_budget)
   int stall_plane = -1;              // forward plane whose copies are withheld (aero_inject_sweep_stall)
   bool configured = false;
   int iflags[8] = {};
@@ -608,7 +609,8 @@ PipeFit pipe_fit(const BlockView* hv, int nblk, int C) {
   }
   f.ok = true;
   // Estimate, from timings of single sweeps, in cycles: a plane's step is bound
-  // by its chain (560) or by a group's way through a plane (1700 and 150 per
+  // by its way from plane to plane (560, of which the chain of dependent operations
+  // is 340) or by a group's way through a plane (1700 and 150 per
   // warp, 240 past 11 warps, where registers run out) shared out over the
   // groups; two CTAs on an SM slow each other (1400 and 130 per warp).  A CTA
   // behind a cut starts about 600 after the one before it.
@@ -640,6 +642,11 @@ PipeFit pipe_sa_fit(const BlockView* hv, int nblk, int C) {
 }
 
 // The pipelined sweeps' cluster size by rule: the smallest estimate of pipe_fit.
+// They run wherever a size fits, since no other sweep came close up to that limit
+// (us a step, pipelined against the best of the others): 57^3 with two stages of
+// planes in two turns 1046 / 2021, 129 x 65 x 33 1257 / 2983; in mixed precision 8
+// blocks of 49^3 2017 / 2329, 20 of 42^3 (2.2 CTAs an SM) 2663 / 2914, 64 of 25^3
+// 1427 / 1592, 300 channels of 17 x 9 x 5 229 / 236, 600 of 9 x 9 x 5 248 / 250.
 PipeFit pipe_choose(const BlockView* hv, int nblk) {
   PipeFit best;
   for (int C : {1, 2, 4, 8, 16}) {
@@ -2997,7 +3004,9 @@ int aero_compute_geometry(int with_walldist) {
 }
 
 // Device-timed iterations for benchmarking: each step is one iteration plus the
-// residual norm (the reference computes it every iteration, outinterval = 1).
+// residual norm (the reference computes it every iteration, outinterval = 1), timed
+// as a call of its own: with the primitives that open it, which the further steps
+// of an aero_step call do not compute.
 // With flush_l2 a 256 MiB buffer is overwritten (cudaMemsetAsync, outside the
 // timed interval) before every step so each step starts with a cold L2.
 int aero_step_timed(int nsteps, int flush_l2, double* device_ms) {

@@ -37,6 +37,8 @@ def main(argv=None) -> int:
     ap.add_argument("--warmup", type=int, default=3)
     ap.add_argument("--inviscid", type=int, default=4, help="4 Roe + WENO3, 5 SW + WENO5, 8 WCNS5")
     ap.add_argument("--mixed", action="store_true")
+    ap.add_argument("--sweep-pipeline", type=int, choices=[1, 2, 4, 8, 16], default=0,
+                    help="CTAs per block of the pipelined sweeps (default: the rule's or the autotuner's)")
     ap.add_argument("--sweep-cluster", type=int, default=0, help="CTAs per block of the LU-SGS sweep in place of the pipelined one (0: autotune)")
     ap.add_argument("--sweep-exchange", choices=["l2", "shared", "slab", "shared2"], default=None,
                     help="plane exchange of a cluster sweep (of 8 CTAs unless --sweep-cluster says; default: L2)")
@@ -62,6 +64,8 @@ def main(argv=None) -> int:
             tuning = ""
         else:
             tuning = "" if args.no_autotune else gc.autotune(3)
+        if args.sweep_pipeline:
+            gc.set_sweep_pipeline(args.sweep_pipeline)
         if args.sweep_cluster or args.sweep_exchange:  # (the pipelined sweeps have no exchange to choose)
             gc.set_sweep_cluster(args.sweep_cluster or 8)
         if args.sweep_exchange:

@@ -177,14 +177,14 @@ class GpuCase:
         _lib.check(self.L.aero_set_sa_sweep_cluster(ctypes.c_int(ctas)), "aero_set_sa_sweep_cluster")
 
     def set_poll_budget(self, polls: int) -> None:
-        """aero_set_poll_budget: polls of each bounded wait of the staged LU-SGS
-        sweep (0..2**20, the default); a wait that gives up raises
+        """aero_set_poll_budget: polls of each wait for a plane's records in the
+        pipelined and the staged LU-SGS sweep (0..2**20, the default); a wait that gives up raises
         AERO_ST_TIMEOUT in the status word."""
         _lib.check(self.L.aero_set_poll_budget(ctypes.c_longlong(polls)), "aero_set_poll_budget")
 
     def inject_sweep_stall(self, plane: int) -> None:
-        """aero_inject_sweep_stall: test hook; the staged LU-SGS sweep never
-        issues the copies of forward hyperplane `plane` (-1: off), so its
+        """aero_inject_sweep_stall: test hook; the pipelined (first slab) and
+        the staged LU-SGS sweep never issue the copies of forward hyperplane `plane` (-1: off), so its
         waits run out and the status word gets AERO_ST_TIMEOUT."""
         _lib.check(self.L.aero_inject_sweep_stall(ctypes.c_int(plane)), "aero_inject_sweep_stall")
 

@@ -141,7 +141,7 @@ module aerocfd_gpu
       integer(c_int), value :: ctas
     end function
 
-    ! polls of each bounded wait of the staged LU-SGS sweep (fault-injection
+    ! polls of each wait for a plane's records in the LU-SGS sweeps (fault-injection
     ! hook; default and largest 1048576)
     integer(c_int) function aero_set_poll_budget(polls) bind(C, name="aero_set_poll_budget")
       import :: c_int, c_long_long

@@ -91,7 +91,9 @@ int aero_get_status(unsigned* status);
 /* Where the first cluster-sweep wait that gave up (AERO_ST_TIMEOUT) was, since
  * the last call: out5 = sweep (1: mean-flow bulk exchange, 2: mean-flow slab,
  * 3: SA, pipelined or slab, 4: the pipelined mean-flow sweep or the one-CTA
- * staged one, whose waits have the poll budget of aero_set_poll_budget), block (0-based), the CTA's rank in its cluster, the step
+ * staged one, whose waits have the poll budget of aero_set_poll_budget;
+ * aero_get_sweep_pipeline tells which of two runs), block (0-based), the CTA's
+ * rank in its cluster, the step
  * (plane step of the forward then backward pass) and the wait (1: a plane's
  * values, 2: the downstream slab's progress, 3: the last plane's values);
  * all -1 when none gave up.  Clears the record.  The cluster sweeps bound
@@ -106,7 +108,8 @@ int aero_timeout_site(int* out5);
  * sweep wait that ran out).  aero_get_block_status copies the nblocks words
  * (block m at out[m-1]) without clearing them; aero_clear_block_status clears
  * them.  With aero_set_retirement(1) every step begins by retiring each block
- * whose word is non-zero: no kernel of the step touches it, so its state stays
+ * whose word is non-zero (a field that is bad when a call begins is marked
+ * after that: it takes the call's first step): no kernel of the step touches it, so its state stays
  * as it was after the step that raised the bit, its residual norms count as 0
  * (aero_residual, aero_residual_blocks) and the other blocks advance as if it
  * were not there (their kernels never read another block, halos aside: retire
@@ -325,9 +328,9 @@ int aero_getpri_all(void);
 int aero_step(int nsteps, double* resid_hist, double* dt_minmax);
 
 /* Benchmark form of aero_step: nsteps iterations, each with its residual
- * norm, timed on the device with CUDA events (device_ms = total); with
- * flush_l2 != 0 the L2 cache is overwritten before every step, outside the
- * timed interval. */
+ * norm and, as an aero_step(1) has them, the primitives it opens with, timed
+ * on the device with CUDA events (device_ms = total); with flush_l2 != 0 the
+ * L2 cache is overwritten before every step, outside the timed interval. */
 int aero_step_timed(int nsteps, int flush_l2, double* device_ms);
 
 /* ---- execution options (no counterpart in the reference) ---------------
@@ -335,8 +338,9 @@ int aero_step_timed(int nsteps, int flush_l2, double* device_ms);
  * (iteration, closing primitives, residual) from a CUDA graph captured on its
  * first use; results are those of the launches it replays.
  * aero_autotune(iters): times iters steps for each candidate launch shape
- * (inviscid-flux CTA tile, element-wise / viscous / block-record thread
- * counts, sweep stages, CTAs per block of the LU-SGS sweep), keeps the fastest
+ * (inviscid-flux CTA tile, element-wise and viscous thread counts, CTAs per
+ * block of the pipelined LU-SGS sweeps or, where others run, their CTAs,
+ * exchange, stages and block-record threads), keeps the fastest
  * of each in turn, and restores the
  * solution state (q, nut, q0, dt, amu) it started from; the arithmetic is the
  * same for every shape.  aero_tuning() describes the shapes in use. */
@@ -364,7 +368,7 @@ int aero_set_sweep_pipeline(int ctas);
  * mean flow's, all 0 when other sweeps run; then the CTAs per block of the SA
  * equation's (0: other sweeps). */
 int aero_get_sweep_pipeline(int* out8);
-/* This call selects another sweep instead, by the CTAs that share a block: 1
+/* Selects another mean-flow sweep instead, by the CTAs that share a block: 1
  * (one CTA per block, the records staged in shared memory when its planes fit) or a thread-block
  * cluster of 2, 4 or 8 CTAs, or 16 CTAs (a non-portable cluster size, with
  * the bulk-copy or the slab exchange only; accepted after aero_finish_setup
@@ -398,14 +402,16 @@ int aero_set_register_bound(int on);
  * CTAs (aero_set_sweep_cluster with exchange 1 or 3) prefetch their shares of
  * the plane records into L2.  Results are the same for every choice; aero_autotune chooses it too. */
 int aero_set_sweep_prefetch(int planes);
-/* Polls each bounded wait of the staged LU-SGS sweep (one CTA per block)
- * makes before it gives up, 0..1048576 (the default); each poll may suspend
- * the waiting thread for a short, system-dependent time.  A wait that gives
+/* Polls each wait for a plane's records makes before it gives up, 0..1048576
+ * (the default), in the mean flow's pipelined sweep (where the default means
+ * one second of the GPU's global timer) and in the one-CTA staged sweep; each
+ * poll may suspend the waiting thread for a short, system-dependent time.  A wait that gives
  * up ends the sweep with AERO_ST_TIMEOUT in the status word and leaves the
  * context usable. */
 int aero_set_poll_budget(long long polls);
-/* Fault injection for tests: in every staged LU-SGS sweep the copies of
- * forward hyperplane `plane` (0-based) are never issued, so the waits for
+/* Fault injection for tests: in every pipelined mean-flow sweep and every
+ * one-CTA staged sweep the copies of forward hyperplane `plane` (0-based; of the
+ * first slab of a pipelined block) are never issued, so the waits for
  * them run out and the sweep ends with AERO_ST_TIMEOUT; -1 (default) turns it
  * off.  The iteration's update is then incomplete. */
 int aero_inject_sweep_stall(int plane);

@@ -12,6 +12,7 @@ ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 @pytest.mark.parametrize("args, text", [
     ([], "sweep_exchange=pipelined"),
+    (["--sweep-pipeline", "4"], "sweep_cluster=4 sweep_exchange=pipelined"),
     (["--sweep-exchange", "slab"], "sweep_cluster=8 sweep_exchange=slab"),
     (["--sweep-exchange", "shared", "--sweep-cluster", "4"], "sweep_cluster=4 sweep_exchange=shared"),
     (["--sweep-cluster", "2"], "sweep_cluster=2 sweep_exchange=l2")])
