@@ -130,7 +130,7 @@ int aero_configure(const int* iflags, const double* params);
  * FP64 throughout).  mode 0 (default): FP64 in the reference's operation order.
  * mode 1 (mixed): the WENO3 corrections, the Roe dissipation and the viscous
  * stresses and fluxes in FP32, each formed from FP64 differences around FP64
- * base states, and the off-diagonal 5x5 blocks of the LU-SGS sweeps stored in
+ * base states, and the off-diagonal 5x5 blocks of the LU-SGS sweeps rounded to
  * FP32 (their products and sums are FP64); metrics, the grid Jacobian, rhs,
  * the implicit diagonal, dq, the time step, the viscosity and the residual
  * stay FP64.  Applies to later calls. */
