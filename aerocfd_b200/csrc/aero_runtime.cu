@@ -2088,8 +2088,7 @@ int aero_set_retirement(int on) {
   int rc = need_setup();
   if (rc) return rc;
   if ((on != 0) == g.retire) return AERO_OK;
-  g.retire = on != 0;
-  graph_release();  // the captured step gains or loses the refresh
+  g.retire = on != 0;  // (the refresh runs before the captured step)
   if (!g.retire) {
     const int nb = (int)g.blocks.size();
     std::vector<int> ones(nb, 1);
